@@ -12,12 +12,12 @@
 // Kernel design. The volume term is a tensor product: with B (N x (N+1)) the LGL basis at the
 // Gauss-Legendre points, B' its derivative and W the weights, the quadrature equals
 //   -(a_x K x M x M + a_y M x K x M + a_z M x M x K) u,  K = B'^T W B,  M = B^T W B,
-// applied sum-factorized (six small passes over an element's (N+1)^3 nodes in shared memory).
-// One thread per node, several elements per CTA; each node then adds the flux of every face
-// it lies on (faces 0..5 in order, own outward normal, the neighbour's face node read from
-// global memory), so the result needs no atomics. The mortar kernels (mortar.cu) add the
-// non-conforming lifts in interface order; the mass inverse is fused into the output or the
-// LSRK update.
+// applied sum-factorized (seven one-dimensional products per node line). A thread works on whole
+// lines of N+1 nodes in registers, so the operator entries are warp-uniform constants; every
+// face adds its flux at the nodes it holds (faces x, y, z in order, own outward normal, the
+// neighbour's face node read from global memory), so the result needs no atomics. The mortar
+// kernels (mortar.cu) add the non-conforming lifts in interface order; the mass inverse is fused
+// into the output or the LSRK update.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -33,7 +33,7 @@ namespace drf {
 namespace {
 
 struct AmrBasis {
-    double K[MAXNP * MAXNP], M[MAXNP * MAXNP], w[MAXNP];
+    double K[MAXNP * MAXNP], M[MAXNP * MAXNP], w[MAXNP], iw[MAXNP];  // iw = 1 / w
 };
 __constant__ AmrBasis cAmr[MAXNP + 1];  // per node count
 
@@ -41,36 +41,26 @@ const double AMR_LSRK_A[5] = {0.0, -0.4178904745, -1.192151694643, -1.6977846924
 const double AMR_LSRK_B[5] = {0.1496590219993, 0.3792103129999, 0.8229550293869, 0.6994504559488,
                               0.1530572479681};
 
+constexpr int AMR_NONE = -1, AMR_BOUNDARY = -2;
+
 struct AmrArgs {
     const double *U;
     double *R;              // weak right-hand side (before the mass inverse)
-    const int64_t *nbe;     // [elem][6] conforming neighbour element (or -1)
-    const int8_t *nbk;      // [elem][6] 0 none, 1 conforming, 2 boundary
-    const int8_t *nbf;      // [elem][6] neighbour face
+    // [elem][6] what lies across each face: the conforming neighbour element (its opposite face
+    // of the same axis, as drf_amr_create checks), AMR_NONE or AMR_BOUNDARY; null: no faces
+    const int *nb;
     int64_t n_elem;
     double ax, ay, az;
     int flux;               // 0 central, 1 upwind, 2 Lax-Friedrichs
     // the LSRK stage form (amr_rhs_kernel<NP, true>): the mortar lifts added in the lift
     // kernel's order, then the mass inverse and res = A res + dt (-M^-1 R), Uout = U + B res
     const double *contrib;  // staged mortar lifts (null: no interfaces)
-    const int64_t *lptr;    // lift entries of touched element u: lent[lptr[u] .. lptr[u + 1])
-    const int *lent;        // (interface, slot, face)
-    const int *e2u;         // touched-element index of each element, -1 if none
-    int slots;
+    const int *lptr;        // lift entries of element e: lent[lptr[e] .. lptr[e + 1])
+    const int2 *lent;       // (row of contrib, face)
     double *res, *Uout;
     double A, B, dt;
     int first;
 };
-
-// One node's LSRK45 stage from its weak right-hand side R (before the mass inverse, the
-// diagonal LGL mass w_i w_j w_k): res = A res + dt (-M^-1 R), u += B res.
-__device__ __forceinline__ void amr_lsrk_node(double R, double wi, double wj, double wk, double &res, double &u,
-                                              double A, double B, double dt, int first) {
-    const double rhs = R * (1.0 / (wi * wj * wk));
-    const double rn = (first ? 0.0 : A * res) + dt * (-rhs);
-    res = rn;
-    u = u + B * rn;
-}
 
 __device__ __forceinline__ double amr_flux(int kind, double uL, double uR, double vn) {
     if (kind == 0) return 0.5 * (vn * uL + vn * uR);
@@ -78,136 +68,220 @@ __device__ __forceinline__ double amr_flux(int kind, double uL, double uR, doubl
     return 0.5 * (vn * uL + vn * uR) - 0.5 * fabs(vn) * (uR - uL);
 }
 
-// volume node of face node (it, jt) of face f: normal index at the boundary, tangents in axis order
+// Elements per CTA and CTAs per SM the kernel is compiled for (its register budget). Up to NP = 4:
+// 64 threads and 73 registers, 28 warps an SM; 256-thread CTAs at 80 registers (24 warps) took
+// 910 us a C3 step against 780 us, 128-thread ones at 64 registers (spills) 860 us. NP = 5, 6:
+// 125 and 108 threads (96 base columns at N = 4: 496 us a step, 256-thread CTAs 660 us).
 template <int NP>
-__device__ __forceinline__ int face_node(int f, int it, int jt) {
-    const int axis = f / 2, b = (f % 2) ? NP - 1 : 0;
-    if (axis == 0) return b + NP * (it + NP * jt);
-    if (axis == 1) return it + NP * (b + NP * jt);
-    return it + NP * (jt + NP * b);
+constexpr int amr_epb() {
+    return (NP <= 4 ? 64 : 128) / (NP * NP);
+}
+template <int NP>
+constexpr int amr_min_ctas() {
+    return NP <= 4 ? 14 : (NP == 5 ? 6 : 5);
 }
 
+// NP consecutive doubles of a line: one 32-byte access (a whole sector) at NP = 4, 16-byte pieces
+// at the other even NP (every line starts on a multiple of its own length in 256-byte aligned
+// arrays)
 template <int NP>
-constexpr int amr_epb() {  // elements per CTA: about 256 threads
-    return (256 / (NP * NP * NP)) < 1 ? 1 : 256 / (NP * NP * NP);
-}
-
-// R = volume term + conforming/boundary face lifts, one thread per node. The element's face
-// table and its conforming neighbours' face traces are loaded at the start (each thread takes
-// face-node slots n, n + NP^3, ...) so those global loads overlap the volume passes. STAGE:
-// the node's mortar lifts are added and the LSRK stage applied (U read, Uout written).
-template <int NP, bool STAGE = false>
-__global__ void __launch_bounds__(amr_epb<NP>() * NP * NP * NP) amr_rhs_kernel(AmrArgs a) {
-    constexpr int NP2 = NP * NP, NP3 = NP2 * NP, EPB = amr_epb<NP>(), NFS = 6 * NP2;
-    constexpr int SLOTS = (NFS + NP3 - 1) / NP3;  // face-node slots per thread
-    __shared__ double sU[EPB * NP3], sP[EPB * NP3], sQ[EPB * NP3], s1[EPB * NP3], s2[EPB * NP3];
-    __shared__ double sN[EPB * NFS];                // neighbour face traces [elem][face][node]
-    __shared__ int sNbe[EPB * 6];
-    __shared__ int8_t sK[EPB * 6], sNf[EPB * 6];
-    // the 1D operators in shared memory: lanes index them by their own node (a constant-memory
-    // read with different addresses across a warp is serialised)
-    __shared__ AmrBasis Bs;
-    for (int t = threadIdx.x; t < NP2; t += blockDim.x) {
-        Bs.K[t] = cAmr[NP].K[t];
-        Bs.M[t] = cAmr[NP].M[t];
-        if (t < NP) Bs.w[t] = cAmr[NP].w[t];
+__device__ __forceinline__ void line_load(double *v, const double *src) {
+    if constexpr (NP == 4) {
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                     : "l"(src)
+                     : "memory");
+    } else if constexpr (NP % 2 == 0) {
+#pragma unroll
+        for (int m = 0; m < NP; m += 2) {
+            const double2 d = *reinterpret_cast<const double2 *>(src + m);
+            v[m] = d.x;
+            v[m + 1] = d.y;
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < NP; ++m) v[m] = src[m];
     }
-    const int le = threadIdx.x / NP3, n = threadIdx.x % NP3;
-    const int i = n % NP, j = (n / NP) % NP, k = n / NP2;
+}
+template <int NP>
+__device__ __forceinline__ void line_store(double *dst, const double *v) {
+    if constexpr (NP == 4) {
+        asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                     : "memory");
+    } else if constexpr (NP % 2 == 0) {
+#pragma unroll
+        for (int m = 0; m < NP; m += 2) *reinterpret_cast<double2 *>(dst + m) = make_double2(v[m], v[m + 1]);
+    } else {
+#pragma unroll
+        for (int m = 0; m < NP; ++m) dst[m] = v[m];
+    }
+}
+
+// R = volume term + conforming/boundary face lifts; STAGE: the mortar lifts are added and the
+// LSRK stage applied (U read, Uout written).
+//
+// One thread per line of N+1 nodes: it takes the z line (i, j), then the y line (i, k), then the
+// x line (j, k) of its element, exchanging lines through shared memory. What the volume term
+// leaves ends on x lines, contiguous in memory, which also are the tangent lines of the y and z
+// faces. The neighbours' face nodes are loaded first, in flight during the passes.
+// Memory-bound: a stage reads U and the register and writes both, 32 B a node, and the products
+// are 7 (N+1) FMAs a node. One thread per node instead (operator entries from shared memory, two
+// loads per FMA) was bound by shared memory: C3 (258,624 hexes, N = 3) 378 us a stage, now 135 us
+// (530 MB, 3.9 TB/s); what is left is the latency of the neighbours' loads.
+// Shared lines have an odd pitch, so that the lanes of a half warp (one element at N = 3) meet
+// distinct banks in the y and x reads.
+template <int NP, bool STAGE = false>
+__global__ void __launch_bounds__(amr_epb<NP>() * NP * NP, amr_min_ctas<NP>()) amr_rhs_kernel(const __grid_constant__ AmrArgs a) {
+    constexpr int NP2 = NP * NP, NP3 = NP2 * NP, N = NP - 1, EPB = amr_epb<NP>();
+    constexpr int PJ = NP | 1, PK = NP * PJ, PE = NP * PK;  // pitches of j, k and the element
+    __shared__ double sU[EPB * PE], sP[EPB * PE], sQ[EPB * PE];
+    __shared__ double sw[NP], siw[NP];
+    const AmrBasis &Bs = cAmr[NP];
+    if (threadIdx.x < NP) {
+        sw[threadIdx.x] = Bs.w[threadIdx.x];
+        siw[threadIdx.x] = Bs.iw[threadIdx.x];
+    }
+    __syncthreads();
+    // the threads of an element meet between its passes: a warp holds whole elements at NP = 2, 4
+    auto line_sync = [] {
+        if constexpr (32 % NP2 == 0) __syncwarp();
+        else __syncthreads();
+    };
+    const int le = threadIdx.x / NP2, l = threadIdx.x % NP2, a0 = l % NP, a1 = l / NP;
     const int64_t e = (int64_t)blockIdx.x * EPB + le;
     const bool valid = e < a.n_elem;
-    double *U = sU + le * NP3, *P = sP + le * NP3, *Q = sQ + le * NP3, *T1 = s1 + le * NP3, *T2 = s2 + le * NP3;
-    const double u = valid ? a.U[e * NP3 + n] : 0.0;
-    if (n < 6) {
-        sK[le * 6 + n] = valid ? a.nbk[e * 6 + n] : (int8_t)0;
-        sNbe[le * 6 + n] = valid ? (int)a.nbe[e * 6 + n] : -1;
-        sNf[le * 6 + n] = valid ? a.nbf[e * 6 + n] : (int8_t)0;
+    // what lies across the faces of the x line (j, k) = (a0, a1)
+    int nx0 = AMR_NONE, nxN = AMR_NONE, ny = AMR_NONE, nz = AMR_NONE;
+    if (valid && a.nb) {
+        const int *t = a.nb + 6 * e;
+        nx0 = t[0];
+        nxN = t[1];
+        if (a0 == 0 || a0 == N) ny = t[a0 == 0 ? 2 : 3];
+        if (a1 == 0 || a1 == N) nz = t[a1 == 0 ? 4 : 5];
     }
-    U[n] = u;
-    __syncthreads();
-    // neighbour face traces: loads issued now, stored to shared memory after the volume passes
-    double nv[SLOTS];
+    int lift0 = 0, lift1 = 0;
+    if (STAGE && valid && a.lptr) {
+        lift0 = a.lptr[e];
+        lift1 = a.lptr[e + 1];
+    }
+    double u[NP];
 #pragma unroll
-    for (int sl = 0; sl < SLOTS; ++sl) {
-        const int slot = n + sl * NP3;
-        nv[sl] = 0.0;
-        if (slot < NFS) {
-            const int f = slot / NP2, fn = slot % NP2;
-            if (sK[le * 6 + f] == 1)
-                nv[sl] = a.U[(int64_t)sNbe[le * 6 + f] * NP3 + face_node<NP>(sNf[le * 6 + f], fn % NP, fn / NP)];
+    for (int k = 0; k < NP; ++k) u[k] = valid ? a.U[e * NP3 + l + NP2 * k] : 0.0;
+    double fx0 = 0.0, fxN = 0.0, fy[NP] = {}, fz[NP] = {};
+    const int xo = NP * l;  // the x line's first node
+    if (nx0 >= 0) fx0 = a.U[(int64_t)nx0 * NP3 + xo + N];
+    if (nxN >= 0) fxN = a.U[(int64_t)nxN * NP3 + xo];
+    if (ny >= 0) line_load<NP>(fy, a.U + (int64_t)ny * NP3 + NP * ((a0 == 0 ? N : 0) + NP * a1));
+    if (nz >= 0) line_load<NP>(fz, a.U + (int64_t)nz * NP3 + NP * (a0 + NP * (a1 == 0 ? N : 0)));
+    // z: P = (I x I x M) u, Q = a_z (I x I x K) u
+    double *U = sU + le * PE, *P = sP + le * PE, *Q = sQ + le * PE;
+    const int oz = a0 + PJ * a1;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        double p = 0.0, q = 0.0;
+#pragma unroll
+        for (int m = 0; m < NP; ++m) {
+            p += Bs.M[k * NP + m] * u[m];
+            q += Bs.K[k * NP + m] * u[m];
+        }
+        U[oz + PK * k] = u[k];
+        P[oz + PK * k] = p;
+        Q[oz + PK * k] = a.az * q;
+    }
+    // the register line, in flight during the other two passes
+    double rs[NP] = {};
+    if (STAGE && valid && !a.first) line_load<NP>(rs, a.res + (size_t)e * NP3 + xo);
+    line_sync();
+    // y: P <- (I x M x I) P, Q <- a_y (I x K x I) P + (I x M x I) Q; a thread rewrites its own line
+    {
+        const int oy = a0 + PK * a1;
+        double pl[NP], ql[NP];
+#pragma unroll
+        for (int m = 0; m < NP; ++m) {
+            pl[m] = P[oy + PJ * m];
+            ql[m] = Q[oy + PJ * m];
+        }
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            double t1 = 0.0, t2 = 0.0, t3 = 0.0;
+#pragma unroll
+            for (int m = 0; m < NP; ++m) {
+                t1 += Bs.M[j * NP + m] * pl[m];
+                t2 += Bs.K[j * NP + m] * pl[m];
+                t3 += Bs.M[j * NP + m] * ql[m];
+            }
+            P[oy + PJ * j] = t1;
+            Q[oy + PJ * j] = a.ay * t2 + t3;
         }
     }
-    // z: P = (I x I x M) u, Q = (I x I x K) u
-    double p = 0.0, q = 0.0;
-#pragma unroll
-    for (int m = 0; m < NP; ++m) {
-        const double um = U[i + NP * (j + NP * m)];
-        p += Bs.M[k * NP + m] * um;
-        q += Bs.K[k * NP + m] * um;
-    }
-    P[n] = p;
-    Q[n] = q;
-    __syncthreads();
-    // y: T1 = (I x M x I) P, T2 = (I x K x I) P, U <- (I x M x I) Q
-    double t1 = 0.0, t2 = 0.0, t3 = 0.0;
-#pragma unroll
-    for (int m = 0; m < NP; ++m) {
-        const int nm = i + NP * (m + NP * k);
-        t1 += Bs.M[j * NP + m] * P[nm];
-        t2 += Bs.K[j * NP + m] * P[nm];
-        t3 += Bs.M[j * NP + m] * Q[nm];
-    }
-    __syncthreads();  // every thread has read U (its own node) and P, Q
-    T1[n] = t1;
-    T2[n] = t2;
-    U[n] = t3;
-#pragma unroll
-    for (int sl = 0; sl < SLOTS; ++sl)
-        if (n + sl * NP3 < NFS) sN[le * NFS + n + sl * NP3] = nv[sl];
-    __syncthreads();
-    // x: r = -(a_x (K x I x I) T1 + a_y (M x I x I) T2 + a_z (M x I x I) T3)
-    double vx = 0.0, vy = 0.0, vz = 0.0;
-#pragma unroll
-    for (int m = 0; m < NP; ++m) {
-        const int nm = m + NP * (j + NP * k);
-        vx += Bs.K[i * NP + m] * T1[nm];
-        vy += Bs.M[i * NP + m] * T2[nm];
-        vz += Bs.M[i * NP + m] * U[nm];
-    }
+    line_sync();
     if (!valid) return;
-    double r = -(a.ax * vx + a.ay * vy + a.az * vz);
-    // faces this node lies on, in face order
+    // x: r = -(a_x (K x I x I) P + (M x I x I) Q)
+    double r[NP];
+    {
+        const int ox = PJ * a0 + PK * a1;
+        double pl[NP], ql[NP];
 #pragma unroll
-    for (int f = 0; f < 6; ++f) {
-        const int axis = f / 2;
-        const int idx = axis == 0 ? i : (axis == 1 ? j : k);
-        if (idx != ((f % 2) ? NP - 1 : 0)) continue;
-        const int kd = sK[le * 6 + f];
-        if (kd == 0) continue;
-        const int it = axis == 0 ? j : i, jt = axis == 2 ? j : k;
-        const double vn = ((f % 2) ? 1.0 : -1.0) * (axis == 0 ? a.ax : (axis == 1 ? a.ay : a.az));
-        const double uR = kd == 1 ? sN[le * NFS + f * NP2 + it + NP * jt] : u;
-        r += Bs.w[it] * Bs.w[jt] * amr_flux(a.flux, u, uR, vn);
+        for (int m = 0; m < NP; ++m) {
+            u[m] = U[ox + m];
+            pl[m] = P[ox + m];
+            ql[m] = Q[ox + m];
+        }
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            double vx = 0.0, vq = 0.0;
+#pragma unroll
+            for (int m = 0; m < NP; ++m) {
+                vx += Bs.K[i * NP + m] * pl[m];
+                vq += Bs.M[i * NP + m] * ql[m];
+            }
+            r[i] = -(a.ax * vx + vq);
+        }
     }
+    // the faces of this line's nodes: both x faces at its ends, a y and a z face along it
+    const double wj = sw[a0], wk = sw[a1];
+    if (nx0 != AMR_NONE) r[0] += wj * wk * amr_flux(a.flux, u[0], nx0 >= 0 ? fx0 : u[0], -a.ax);
+    if (nxN != AMR_NONE) r[N] += wj * wk * amr_flux(a.flux, u[N], nxN >= 0 ? fxN : u[N], a.ax);
+    if (ny != AMR_NONE) {
+        const double vn = a0 == 0 ? -a.ay : a.ay;
+#pragma unroll
+        for (int i = 0; i < NP; ++i) r[i] += Bs.w[i] * wk * amr_flux(a.flux, u[i], ny >= 0 ? fy[i] : u[i], vn);
+    }
+    if (nz != AMR_NONE) {
+        const double vn = a1 == 0 ? -a.az : a.az;
+#pragma unroll
+        for (int i = 0; i < NP; ++i) r[i] += Bs.w[i] * wj * amr_flux(a.flux, u[i], nz >= 0 ? fz[i] : u[i], vn);
+    }
+    const size_t t = (size_t)e * NP3 + xo;
     if constexpr (STAGE) {
         // mortar lifts of the interfaces touching this element, in the lift kernel's order
-        const int ut = a.e2u ? a.e2u[e] : -1;
-        if (ut >= 0)
-            for (int64_t q = a.lptr[ut]; q < a.lptr[ut + 1]; ++q) {
-                const int iface = a.lent[3 * q], slot = a.lent[3 * q + 1], f = a.lent[3 * q + 2];
-                const int axis = f >> 1, b = (f & 1) ? NP - 1 : 0;
-                const int on = axis == 0 ? i : (axis == 1 ? j : k);
-                if (on != b) continue;
-                const int it = axis == 0 ? j : i, jt = axis == 2 ? j : k;
-                r += a.contrib[((size_t)iface * a.slots + slot) * NP2 + it + NP * jt];
+        for (int q = lift0; q < lift1; ++q) {
+            const int2 en = a.lent[q];
+            const double *c = a.contrib + (size_t)en.x * NP2;
+            const int f = en.y, b = (f & 1) ? N : 0;
+            if (f < 2) {
+                const double v = c[l];
+                if (b == 0) r[0] += v;
+                else r[N] += v;
+            } else if ((f < 4 ? a0 : a1) == b) {
+                double v[NP];
+                line_load<NP>(v, c + NP * (f < 4 ? a1 : a0));
+#pragma unroll
+                for (int i = 0; i < NP; ++i) r[i] += v[i];
             }
-        const size_t t = (size_t)e * NP3 + n;
-        double rs = a.first ? 0.0 : a.res[t], uo = u;
-        amr_lsrk_node(r, Bs.w[i], Bs.w[j], Bs.w[k], rs, uo, a.A, a.B, a.dt, a.first);
-        a.res[t] = rs;
-        a.Uout[t] = uo;
+        }
+        // the LSRK45 stage from the weak right-hand side (mass w_i w_j w_k):
+        // res = A res + dt (-M^-1 R), u += B res
+        const double im = siw[a0] * siw[a1];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            rs[i] = (a.first ? 0.0 : a.A * rs[i]) - a.dt * (r[i] * (im * Bs.iw[i]));
+            u[i] += a.B * rs[i];
+        }
+        line_store<NP>(a.res + t, rs);
+        line_store<NP>(a.Uout + t, u);
     } else {
-        a.R[e * NP3 + n] = r;
+        line_store<NP>(a.R + t, r);
     }
 }
 
@@ -426,14 +500,14 @@ struct drf_amr {
     int order = 0, np = 0, nd = 0;
     int64_t n_elem = 0, n_conf = 0, n_bnd = 0, n_if = 0;
     cudaStream_t stream = nullptr, own = nullptr;
-    DevBuf<int64_t> nbe;
-    DevBuf<int8_t> nbk, nbf;
+    DevBuf<int> nb;  // what lies across each element's faces (AmrArgs::nb)
     // device state (two buffers: an LSRK stage reads one and writes the other; cur holds the
     // state between steps), weak rhs, LSRK register, caller-visible rhs
     DevBuf<double> U, R, res, out;
     int cur = 0;
     drf_mortar *mortar = nullptr;
-    DevBuf<int> e2u;  // touched-element index of each element for the stage kernel's lifts
+    DevBuf<int> lptr;   // the stage kernel's mortar lifts per element (AmrArgs::lptr, lent)
+    DevBuf<int2> lent;
     // step graphs for each starting buffer (a step's five stages flip it)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     uint64_t graph_kernels = 0;  // kernel nodes of a step graph
@@ -457,14 +531,13 @@ struct drf_amr {
     // R = weak right-hand side of U (volume + faces of the mode + mortar lifts)
     void enqueue_rhs(int mode, int flux, const double a[3]) {
         AmrArgs A{};
-        A.U = state(); A.R = R.p; A.nbe = nbe.p; A.nbf = nbf.p; A.n_elem = n_elem;
+        A.U = state(); A.R = R.p; A.n_elem = n_elem;
         A.ax = a[0]; A.ay = a[1]; A.az = a[2]; A.flux = flux;
-        // mode 0 reads an all-zero face table: the reference's TODO branches
-        A.nbk = mode == 1 ? nbk.p : nbk.p + (size_t)6 * n_elem;
+        A.nb = mode == 1 ? nb.p : nullptr;  // mode 0: the reference's TODO branches
         amr_dispatch(np, [&](auto npc) {
             constexpr int NP = decltype(npc)::value;
             constexpr int EPB = amr_epb<NP>();
-            amr_rhs_kernel<NP><<<(unsigned)((n_elem + EPB - 1) / EPB), EPB * NP * NP * NP, 0, stream>>>(A);
+            amr_rhs_kernel<NP><<<(unsigned)((n_elem + EPB - 1) / EPB), EPB * NP * NP, 0, stream>>>(A);
             DRF_LAUNCHED();
         });
         if (mortar) {
@@ -481,17 +554,18 @@ struct drf_amr {
             if (mortar) mortar_stage_faces(mortar, flux, a, buf(src));
             AmrArgs A{};
             A.U = buf(src); A.Uout = buf(1 - src); A.res = res.p;
-            A.nbe = nbe.p; A.nbf = nbf.p; A.n_elem = n_elem;
-            A.nbk = mode == 1 ? nbk.p : nbk.p + (size_t)6 * n_elem;
+            A.nb = mode == 1 ? nb.p : nullptr;
+            A.n_elem = n_elem;
             A.ax = a[0]; A.ay = a[1]; A.az = a[2]; A.flux = flux;
-            A.contrib = mortar ? L.contrib : nullptr; A.lptr = L.ptr; A.lent = L.ent;
-            A.e2u = mortar ? e2u.p : nullptr; A.slots = L.slots;
+            A.contrib = mortar ? L.contrib : nullptr;
+            A.lptr = mortar ? lptr.p : nullptr;
+            A.lent = lent.p;
             A.A = AMR_LSRK_A[s]; A.B = AMR_LSRK_B[s]; A.dt = dt; A.first = s == 0;
             amr_dispatch(np, [&](auto npc) {
                 constexpr int NP = decltype(npc)::value;
                 constexpr int EPB = amr_epb<NP>();
                 amr_rhs_kernel<NP, true>
-                    <<<(unsigned)((n_elem + EPB - 1) / EPB), EPB * NP * NP * NP, 0, stream>>>(A);
+                    <<<(unsigned)((n_elem + EPB - 1) / EPB), EPB * NP * NP, 0, stream>>>(A);
                 DRF_LAUNCHED();
             });
         }
@@ -562,6 +636,7 @@ void upload_amr_basis(int order) {
     std::memset(&ab, 0, sizeof(ab));
     for (int i = 0; i < np; ++i) {
         ab.w[i] = b.w[i];
+        ab.iw[i] = 1.0 / b.w[i];
         for (int m = 0; m < np; ++m) {
             double k = 0.0, mm = 0.0;
             for (int q = 0; q < nq; ++q) {
@@ -598,34 +673,26 @@ int drf_amr_create(int order, int64_t n_elem, int64_t n_conf, const int64_t *con
         h->n_conf = n_conf;
         h->n_bnd = n_bnd;
         h->n_if = n_if;
-        // face table: the second half stays zero (the reference-semantics launches read it)
-        std::vector<int64_t> nbe((size_t)6 * n_elem, -1);
-        std::vector<int8_t> nbk((size_t)12 * n_elem, 0), nbf((size_t)6 * n_elem, 0);
-        auto set = [&](int64_t e, int64_t f, int8_t kd, int64_t e2, int64_t f2) {
+        std::vector<int> nb((size_t)6 * n_elem, AMR_NONE);
+        auto set = [&](int64_t e, int64_t f, int64_t across) {
             DRF_CHECK(e >= 0 && e < n_elem && f >= 0 && f < 6, DRF_E_INVALID, "face list entry out of range");
-            DRF_CHECK(nbk[e * 6 + f] == 0, DRF_E_INVALID, "face listed twice");
-            nbk[e * 6 + f] = kd;
-            nbe[e * 6 + f] = e2;
-            nbf[e * 6 + f] = (int8_t)f2;
+            DRF_CHECK(nb[e * 6 + f] == AMR_NONE, DRF_E_INVALID, "face listed twice");
+            nb[e * 6 + f] = (int)across;
         };
         for (int64_t i = 0; i < n_conf; ++i) {
             const int64_t *c = conf + 4 * i;
             DRF_CHECK(c[2] >= 0 && c[2] < n_elem && c[3] >= 0 && c[3] < 6 && c[1] / 2 == c[3] / 2 &&
                           c[1] != c[3],
                       DRF_E_INVALID, "conforming pair must join opposite faces of one axis");
-            set(c[0], c[1], 1, c[2], c[3]);
-            set(c[2], c[3], 1, c[0], c[1]);
+            set(c[0], c[1], c[2]);
+            set(c[2], c[3], c[0]);
         }
-        for (int64_t i = 0; i < n_bnd; ++i) set(bnd[2 * i], bnd[2 * i + 1], 2, -1, 0);
+        for (int64_t i = 0; i < n_bnd; ++i) set(bnd[2 * i], bnd[2 * i + 1], AMR_BOUNDARY);
         upload_amr_basis(order);
         DRF_CUDA(cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking));
         h->stream = h->own;
-        h->nbe.alloc(nbe.size());
-        h->nbk.alloc(nbk.size());
-        h->nbf.alloc(nbf.size());
-        DRF_CUDA(cudaMemcpy(h->nbe.p, nbe.data(), nbe.size() * 8, cudaMemcpyHostToDevice));
-        DRF_CUDA(cudaMemcpy(h->nbk.p, nbk.data(), nbk.size(), cudaMemcpyHostToDevice));
-        DRF_CUDA(cudaMemcpy(h->nbf.p, nbf.data(), nbf.size(), cudaMemcpyHostToDevice));
+        h->nb.alloc(nb.size());
+        DRF_CUDA(cudaMemcpy(h->nb.p, nb.data(), nb.size() * sizeof(int), cudaMemcpyHostToDevice));
         const size_t n = (size_t)n_elem * h->nd;
         h->U.alloc(2 * n);
         h->R.alloc(n);
@@ -638,15 +705,23 @@ int drf_amr_create(int order, int64_t n_elem, int64_t n_conf, const int64_t *con
                                              n_elem, &h->mortar);
             DRF_CHECK(rc == DRF_OK, rc, "mortar interfaces rejected");
             DRF_CHECK(drf_mortar_set_stream(h->mortar, h->stream) == DRF_OK, DRF_E_CUDA, "mortar stream");
-            // each element's index in the mortar space's touched-element list (-1: none)
+            // the mortar space's lift lists by element
             const MortarLifts L = mortar_lifts(h->mortar);
-            std::vector<int64_t> touched((size_t)std::max<int64_t>(L.n_touched, 1));
-            if (L.n_touched > 0)
-                DRF_CUDA(cudaMemcpy(touched.data(), L.touched, L.n_touched * 8, cudaMemcpyDeviceToHost));
-            std::vector<int> e2u((size_t)n_elem, -1);
-            for (int64_t u = 0; u < L.n_touched; ++u) e2u[touched[u]] = (int)u;
-            h->e2u.alloc(n_elem);
-            DRF_CUDA(cudaMemcpy(h->e2u.p, e2u.data(), n_elem * 4, cudaMemcpyHostToDevice));
+            std::vector<int64_t> touched(L.n_touched), ptr(L.n_touched + 1);
+            DRF_CUDA(cudaMemcpy(touched.data(), L.touched, L.n_touched * 8, cudaMemcpyDeviceToHost));
+            DRF_CUDA(cudaMemcpy(ptr.data(), L.ptr, ptr.size() * 8, cudaMemcpyDeviceToHost));
+            std::vector<int> ent(3 * (size_t)ptr.back()), lp((size_t)n_elem + 1, 0);
+            DRF_CUDA(cudaMemcpy(ent.data(), L.ent, ent.size() * 4, cudaMemcpyDeviceToHost));
+            DRF_CHECK(n_if * L.slots < ((int64_t)1 << 31), DRF_E_UNSUPPORTED, "AMR: too many interfaces");
+            std::vector<int2> le((size_t)ptr.back());
+            for (size_t q = 0; q < le.size(); ++q)
+                le[q] = make_int2(ent[3 * q] * L.slots + ent[3 * q + 1], ent[3 * q + 2]);
+            for (int64_t u = 0; u < L.n_touched; ++u) lp[touched[u] + 1] = (int)(ptr[u + 1] - ptr[u]);
+            for (int64_t e = 0; e < n_elem; ++e) lp[e + 1] += lp[e];
+            h->lptr.alloc(lp.size());
+            h->lent.alloc(le.size());
+            DRF_CUDA(cudaMemcpy(h->lptr.p, lp.data(), lp.size() * 4, cudaMemcpyHostToDevice));
+            DRF_CUDA(cudaMemcpy(h->lent.p, le.data(), le.size() * sizeof(int2), cudaMemcpyHostToDevice));
         }
         *out = h.release();
     });

@@ -11,7 +11,7 @@
 //    reference); P = M^-1 B, L = B^T for both sides;
 //  * flux at mortar node m from (P_c U_c)_m and (sum_f P_f U_f)_m with the coarse face's
 //    outward axis normal; coarse lift L_c M^-1 F, fine lifts -L_f M^-1 F.
-// Device work: one warp per interface computes all lifted face values into a staging buffer;
+// Device work: one thread per mortar node computes all lifted face values into a staging buffer;
 // a second kernel adds them into the element right-hand sides, one thread per element node,
 // in interface order (deterministic, no atomics).
 #include <algorithm>
@@ -28,9 +28,7 @@ namespace drf {
 namespace {
 
 constexpr int MORTAR_TYPES = 6;  // FaceConnectionType SameLevel .. Fine2x2 (face_connection.hpp:15)
-constexpr int MAXNM = MAXNP * MAXNP;
 constexpr int SLOTS = 5;         // coarse side + up to 4 fine faces
-constexpr int MW = 8;            // warps per CTA of the face kernel
 
 int type_num_fine(int t) {
     static const int n[MORTAR_TYPES] = {1, 2, 2, 3, 3, 4};
@@ -192,15 +190,54 @@ HostOps build_ops(int order, int t) {
     return o;
 }
 
-// device operator block of one type: Minv | Pc | Lc | Pf[4] | Lf[4], each nm * nm doubles,
-// stored transposed (column-major)
-constexpr int OPS_MATS = 11;
-__host__ __device__ inline size_t ops_stride(int nm) { return (size_t)OPS_MATS * nm * nm; }
+// The fine coupling of every type is a tensor product: the quadrature points inside a sub-face
+// rectangle are a product of two 1D sets, so P_f = M^-1 B_f = P2 x P1 with P1, P2 the 1D
+// projections of the whole edge (the identity: B = M there) or of its lower or upper half, and
+// the lift L_f M^-1 = B_f^T M^-1 = P_f^T; on the coarse side P_c = I and L_c M^-1 = I.
+// sub_half(t, f): which part of the edge along t1 and t2 sub-face f of type t covers (0 the
+// whole edge, 1 its lower and 2 its upper half), t1 in bits 0-1 and t2 in bits 2-3, as
+// subface_bounds lists them.
+__device__ __forceinline__ int sub_half(int t, int f) {
+    // one byte a sub-face, f = 0 in the low byte
+    const unsigned tab = t == 0 ? 0x00000000u : t == 1 ? 0x00000201u : t == 2 ? 0x00000804u
+                       : t == 3 ? 0x00080605u : t == 4 ? 0x00020905u : 0x0a090605u;
+    return (tab >> (8 * f)) & 15;
+}
+
+// 1D projections of a half edge onto the mortar nodes, H[lower, upper][np][np] row-major:
+// (M1^-1 B1)[m][j], B1 over the quadrature points inside the closed half (a point on the split
+// belongs to both halves, as in the reference)
+std::vector<double> half_edge_ops(int order) {
+    const HostBasis lgl = make_lgl_basis(order);
+    const int np = order + 1, nq = 2 * order + 1;
+    std::vector<double> gx, gw, M((size_t)np * np, 0.0), H((size_t)2 * np * np, 0.0);
+    gauss_legendre(nq, gx, gw);
+    std::vector<double> phi((size_t)nq * np), ps(np);
+    for (int q = 0; q < nq; ++q) lagrange(lgl.x, gx[q], &phi[q * np]);
+    for (int q = 0; q < nq; ++q)
+        for (int m = 0; m < np; ++m)
+            for (int j = 0; j < np; ++j) M[m * np + j] += gw[q] * phi[q * np + m] * phi[q * np + j];
+    const std::vector<double> Mi = inverse(M, np);
+    for (int s = 0; s < 2; ++s) {
+        const double lo = s == 0 ? -1.0 : 0.0, hi = s == 0 ? 0.0 : 1.0;
+        std::vector<double> B((size_t)np * np, 0.0);
+        for (int q = 0; q < nq; ++q) {
+            if (!(gx[q] >= lo && gx[q] <= hi)) continue;
+            lagrange(lgl.x, 2.0 * (gx[q] - lo) / (hi - lo) - 1.0, ps.data());
+            for (int m = 0; m < np; ++m)
+                for (int j = 0; j < np; ++j) B[m * np + j] += gw[q] * phi[q * np + m] * ps[j];
+        }
+        for (int r = 0; r < np; ++r)
+            for (int k = 0; k < np; ++k)
+                for (int c = 0; c < np; ++c) H[(size_t)(s * np + r) * np + c] += Mi[r * np + k] * B[k * np + c];
+    }
+    return H;
+}
 
 struct MortarDev {
-    int np, nm, nd;
+    int nd;
     int64_t n_if;
-    const double *ops;                 // MORTAR_TYPES blocks of ops_stride(nm)
+    const double *H;                   // half-edge projections [2][np][np]
     const int *type, *cface, *fface;   // fface: 4 per interface
     const int64_t *celem, *felem;      // felem: 4 per interface
 };
@@ -222,66 +259,84 @@ __device__ __forceinline__ double scalar_flux(int kind, double uL, double uR, do
     return 0.5 * (vn * uL + vn * uR) - 0.5 * fabs(vn) * (uR - uL);
 }
 
-// NP (nodes per direction) is a compile-time constant so the small dense products unroll and
-// their operator loads pipeline.
+// Every interface's lifts into contrib[interface][slot][face node]. One thread per mortar node
+// (it, jt), several interfaces a CTA; a sub-face takes one or two 1D products of NP terms per
+// node in each direction (up for its trace, down for its lift) through shared memory.
+// The dense form of the same operators (a warp per interface, NP^2 terms a product, operators
+// from global memory) took 69 us for C3's 25,506 interfaces, this one 20 us; the traces and lifts are 33 MB.
 template <int NP>
-__global__ void __launch_bounds__(32 * MW) mortar_face_kernel(MortarDev D, int kind, double a0, double a1,
-                                                              double a2, const double *__restrict__ U,
-                                                              double *__restrict__ contrib) {
-    constexpr int nm = NP * NP, nf = NP * NP, np = NP;
-    __shared__ double sU[MW][SLOTS][nm];
-    __shared__ double sF[MW][nm], sG[MW][nm];
-    const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
-    for (int64_t i = blockIdx.x * (int64_t)MW + w; i < D.n_if; i += (int64_t)gridDim.x * MW) {
-        const int t = D.type[i], nfine = type_num_fine_dev(t);
-        const double *op = D.ops + (size_t)t * ops_stride(nm);
-        const double *Minv = op, *Pc = op + nm * nm, *Lc = op + 2 * nm * nm;
-        const double *Pf = op + 3 * nm * nm, *Lf = op + 7 * nm * nm;
-        const int cf = D.cface[i];
-        for (int j = lane; j < nf; j += 32) {
-            sU[w][0][j] = U[D.celem[i] * D.nd + face_node(np, cf, j % np, j / np)];
-            for (int f = 0; f < nfine; ++f)
-                sU[w][1 + f][j] = U[D.felem[4 * i + f] * D.nd + face_node(np, D.fface[4 * i + f], j % np, j / np)];
+constexpr int mortar_ipb() {  // interfaces per CTA: about 128 threads
+    return 128 / (NP * NP);
+}
+template <int NP>
+__global__ void __launch_bounds__(mortar_ipb<NP>() * NP * NP)
+    mortar_face_kernel(MortarDev D, int kind, double a0, double a1, double a2, const double *__restrict__ U,
+                       double *__restrict__ contrib) {
+    constexpr int nm = NP * NP, IPB = mortar_ipb<NP>();
+    __shared__ double sH[2][NP][NP];
+    __shared__ double sA[IPB][4][nm], sB[IPB][4][nm], sF[IPB][nm];
+    for (int q = threadIdx.x; q < 2 * nm; q += IPB * nm) (&sH[0][0][0])[q] = D.H[q];
+    const int w = threadIdx.x / nm, m = threadIdx.x % nm, it = m % NP, jt = m / NP;
+    const int64_t i = blockIdx.x * (int64_t)IPB + w;
+    const bool valid = i < D.n_if;
+    const int t = valid ? D.type[i] : 0, nfine = valid ? type_num_fine_dev(t) : 0;
+    const int cf = valid ? D.cface[i] : 0;
+    double uc = 0.0;
+    if (valid) {
+        uc = U[D.celem[i] * D.nd + face_node(NP, cf, it, jt)];
+        for (int f = 0; f < nfine; ++f)
+            sA[w][f][m] = U[D.felem[4 * i + f] * D.nd + face_node(NP, D.fface[4 * i + f], it, jt)];
+    }
+    __syncthreads();
+    for (int f = 0; f < nfine; ++f) {  // along t1
+        const int h = sub_half(t, f) & 3;
+        double s = sA[w][f][m];
+        if (h) {
+            s = 0.0;
+#pragma unroll
+            for (int k = 0; k < NP; ++k) s += sH[h - 1][it][k] * sA[w][f][k + NP * jt];
         }
-        __syncwarp();
-        const int axis = cf >> 1;
-        const double vn = ((cf & 1) ? 1.0 : -1.0) * (axis == 0 ? a0 : (axis == 1 ? a1 : a2));
-        for (int m = lane; m < nm; m += 32) {
-            double uc = 0.0, uf = 0.0;
+        sB[w][f][m] = s;
+    }
+    __syncthreads();
+    double uf = 0.0;
+    for (int f = 0; f < nfine; ++f) {  // along t2, summed over the sub-faces
+        const int h = sub_half(t, f) >> 2;
+        double s = sB[w][f][m];
+        if (h) {
+            s = 0.0;
 #pragma unroll
-            for (int j = 0; j < nf; ++j) uc += Pc[j * nm + m] * sU[w][0][j];
-            for (int f = 0; f < nfine; ++f) {
-                double s = 0.0;
-                const double *P = Pf + (size_t)f * nm * nm + m;
-#pragma unroll
-                for (int j = 0; j < nf; ++j) s += P[j * nm] * sU[w][1 + f][j];
-                uf += s;
-            }
-            sF[w][m] = scalar_flux(kind, uc, uf, vn);
+            for (int k = 0; k < NP; ++k) s += sH[h - 1][jt][k] * sB[w][f][it + NP * k];
         }
-        __syncwarp();
-        for (int m = lane; m < nm; m += 32) {
-            double g = 0.0;
+        uf += s;
+    }
+    const int axis = cf >> 1;
+    const double vn = ((cf & 1) ? 1.0 : -1.0) * (axis == 0 ? a0 : (axis == 1 ? a1 : a2));
+    const double F = scalar_flux(kind, uc, uf, vn);
+    sF[w][m] = F;
+    __syncthreads();
+    double *out = contrib + (size_t)i * SLOTS * nm;
+    if (valid) out[m] = F;
+    for (int f = 0; f < nfine; ++f) {  // P_f^T F: along t1
+        const int h = sub_half(t, f) & 3;
+        double s = F;
+        if (h) {
+            s = 0.0;
 #pragma unroll
-            for (int k = 0; k < nm; ++k) g += Minv[k * nm + m] * sF[w][k];
-            sG[w][m] = g;
+            for (int k = 0; k < NP; ++k) s += sH[h - 1][k][it] * sF[w][k + NP * jt];
         }
-        __syncwarp();
-        double *out = contrib + (size_t)i * SLOTS * nf;
-        for (int j = lane; j < nf; j += 32) {
-            double s = 0.0;
+        sA[w][f][m] = s;
+    }
+    __syncthreads();
+    for (int f = 0; f < nfine; ++f) {  // along t2
+        const int h = sub_half(t, f) >> 2;
+        double s = sA[w][f][m];
+        if (h) {
+            s = 0.0;
 #pragma unroll
-            for (int m = 0; m < nm; ++m) s += Lc[m * nf + j] * sG[w][m];
-            out[j] = s;
-            for (int f = 0; f < nfine; ++f) {
-                const double *L = Lf + (size_t)f * nm * nm + j;
-                double sf = 0.0;
-#pragma unroll
-                for (int m = 0; m < nm; ++m) sf += L[m * nf] * sG[w][m];
-                out[(1 + f) * nf + j] = -sf;
-            }
+            for (int k = 0; k < NP; ++k) s += sH[h - 1][k][jt] * sA[w][f][it + NP * k];
         }
-        __syncwarp();
+        out[(1 + f) * nm + m] = -s;
     }
 }
 
@@ -324,7 +379,7 @@ struct drf_mortar {
     int order = 0, np = 0, nm = 0, nd = 0;
     int64_t n_if = 0, n_elem = 0, n_touched = 0;
     cudaStream_t stream = nullptr, own = nullptr;
-    DevBuf<double> ops, contrib, U, rhs;
+    DevBuf<double> half, contrib, U, rhs;
     DevBuf<int> type, cface, fface, ent;
     DevBuf<int64_t> celem, felem, touched, ptr;
     ~drf_mortar() {
@@ -332,8 +387,8 @@ struct drf_mortar {
     }
     MortarDev dev() const {
         MortarDev D;
-        D.np = np; D.nm = nm; D.nd = nd; D.n_if = n_if;
-        D.ops = ops.p; D.type = type.p; D.cface = cface.p; D.fface = fface.p;
+        D.nd = nd; D.n_if = n_if;
+        D.H = half.p; D.type = type.p; D.cface = cface.p; D.fface = fface.p;
         D.celem = celem.p; D.felem = felem.p;
         return D;
     }
@@ -347,13 +402,17 @@ struct drf_mortar {
     }
     void stage_faces(int kind, const double a[3], const double *dU) {
         if (n_if == 0) return;
-        const unsigned g = (unsigned)std::min<int64_t>((n_if + MW - 1) / MW, 148 * 16);
+        auto launch = [&](auto npc) {
+            constexpr int NP = decltype(npc)::value, IPB = mortar_ipb<NP>();
+            mortar_face_kernel<NP><<<(unsigned)((n_if + IPB - 1) / IPB), IPB * NP * NP, 0, stream>>>(
+                dev(), kind, a[0], a[1], a[2], dU, contrib.p);
+        };
         switch (np) {
-        case 2: mortar_face_kernel<2><<<g, 32 * MW, 0, stream>>>(dev(), kind, a[0], a[1], a[2], dU, contrib.p); break;
-        case 3: mortar_face_kernel<3><<<g, 32 * MW, 0, stream>>>(dev(), kind, a[0], a[1], a[2], dU, contrib.p); break;
-        case 4: mortar_face_kernel<4><<<g, 32 * MW, 0, stream>>>(dev(), kind, a[0], a[1], a[2], dU, contrib.p); break;
-        case 5: mortar_face_kernel<5><<<g, 32 * MW, 0, stream>>>(dev(), kind, a[0], a[1], a[2], dU, contrib.p); break;
-        default: mortar_face_kernel<6><<<g, 32 * MW, 0, stream>>>(dev(), kind, a[0], a[1], a[2], dU, contrib.p); break;
+        case 2: launch(std::integral_constant<int, 2>{}); break;
+        case 3: launch(std::integral_constant<int, 3>{}); break;
+        case 4: launch(std::integral_constant<int, 4>{}); break;
+        case 5: launch(std::integral_constant<int, 5>{}); break;
+        default: launch(std::integral_constant<int, 6>{}); break;
         }
         DRF_LAUNCHED();
     }
@@ -425,27 +484,7 @@ int drf_mortar_create(int order, int64_t n_if, const int *type, const int64_t *c
         h->nd = h->np * h->nm;
         h->n_if = n_if;
         h->n_elem = n_elem;
-        // operators of every connection type
-        std::vector<double> ops(MORTAR_TYPES * ops_stride(h->nm), 0.0);
-        for (int t = 0; t < MORTAR_TYPES; ++t) {
-            const HostOps o = build_ops(order, t);
-            double *dst = ops.data() + t * ops_stride(h->nm);
-            const int nm = h->nm;
-            const size_t n2 = (size_t)nm * nm;
-            // stored transposed: in the face kernel lane m reads row m, so column-major storage
-            // makes a warp's reads of one column consecutive addresses
-            auto put_t = [&](double *d, const std::vector<double> &A) {
-                for (int r = 0; r < nm; ++r)
-                    for (int c = 0; c < nm; ++c) d[(size_t)c * nm + r] = A[(size_t)r * nm + c];
-            };
-            put_t(dst, o.Minv);
-            put_t(dst + n2, o.Pc);
-            put_t(dst + 2 * n2, o.Lc);
-            for (int f = 0; f < o.nfine; ++f) {
-                put_t(dst + (3 + f) * n2, o.Pf[f]);
-                put_t(dst + (7 + f) * n2, o.Lf[f]);
-            }
-        }
+        const std::vector<double> half = half_edge_ops(order);
         // interfaces, validated; per-element entries in interface order
         std::vector<int> ty(n_if), cf(n_if), ff(4 * n_if, 0);
         std::vector<int64_t> ce(n_if), fe(4 * n_if, 0);
@@ -480,7 +519,7 @@ int drf_mortar_create(int order, int64_t n_if, const int *type, const int64_t *c
         h->n_touched = (int64_t)touched.size();
         DRF_CUDA(cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking));
         h->stream = h->own;
-        upload(h->ops, ops);
+        upload(h->half, half);
         upload(h->type, ty); upload(h->cface, cf); upload(h->fface, ff);
         upload(h->celem, ce); upload(h->felem, fe);
         upload(h->touched, touched); upload(h->ptr, ptr); upload(h->ent, ent);

@@ -76,6 +76,30 @@ def test_lsrk_steps_match_oracle(small, mode):
     gpu.close()
 
 
+@pytest.mark.parametrize("order", [1, 2, 4, 5])
+@pytest.mark.parametrize("mesh", ["coast", "uniform"])
+def test_lsrk_steps_other_orders(order, mesh):
+    """The stage kernel at the other orders: element counts that leave the last CTA part empty, and
+    a mesh without interfaces (3 x 5 columns, two layers). Tolerance: an FP64 step of at most
+    sums of 7 (N + 1) products a node, in another order than the oracle's."""
+    if mesh == "coast":
+        c = configs.c3(nb=7, order=order)
+        m, U = c["mesh"], c["U"]
+    else:
+        from drifter_b200.amr import build_mesh
+        z = np.zeros((5, 3), np.int32)
+        m = build_mesh(z, z, z + 1)
+        assert m["n_elem"] == 30 and len(m["ifaces"]) == 0
+        U = np.random.default_rng(order).standard_normal((30, (order + 1) ** 3))
+    a, dt = np.array([0.7, -0.4, 0.9]), 1e-4
+    gpu = DG3DIntegration(order, m)
+    gpu.upload(U)
+    gpu.step(a, dt, 2, flux="lf", mode="complete")
+    r = O.amr_lsrk(order, m, 1, 2, a, U, dt, 2)
+    assert relerr(gpu.download(), r) < 1e-12
+    gpu.close()
+
+
 def test_bad_inputs_are_rejected(small):
     m = small["mesh"]
     gpu = DG3DIntegration(3, m)
