@@ -1203,8 +1203,62 @@ __device__ __forceinline__ void lf_minus_phys(const double UL[3], double ihL, do
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         const double FnL = FxL[q] * nx + FyL[q] * ny, FnR = FxR[q] * nx + FyR[q] * ny;
-        d[q] = (0.5 * (FnL + FnR) - 0.5 * lam * (UR[q] - UL[q])) - Fm[q];
+        d[q] = __fma_rn(0.5, FnL + FnR, -__dmul_rn(__dmul_rn(0.5, lam), UR[q] - UL[q])) - Fm[q];
     }
+}
+
+// d = F*(U-, U+, n) - F(U-).n for a face normal along an axis, in the face's own components:
+// U = (h, hn, ht) with hn, ht the momentum along and across the axis, sg = +-1 the outward
+// direction along it, iL = 1 / h- (clamped as below). The interior flux is taken out of F*
+// algebraically, which also takes out the cancellation of their 0.5 g h^2. Same states, speeds and
+// branches as sw_flux; one division per state and speed instead of seven and more (23 x 17 columns at
+// N = 2 with HLLC, resident form: 178 us a step against 208 us with F* and F- formed separately).
+__device__ __forceinline__ double wet(double h) { return h < 1e-10 ? 1e-10 : h; }
+template <int FK>
+__device__ __forceinline__ void axis_flux_diff(const double L[3], double iL, const double R[3], double sg, double g,
+                                               double d[3]) {
+    const double hL = wet(L[0]), hR = wet(R[0]), iR = 1.0 / hR;
+    const double nL = sg * L[1], nR = sg * R[1];  // outward momenta
+    const double uL = nL * iL, uR = nR * iR;      // outward velocities
+    const double vL = L[2] * iL, vR = R[2] * iR;
+    const double dh = R[0] - L[0], dn = nR - nL, dt = R[2] - L[2];
+    const double cR = sqrt(g * hR), cL = sqrt(g * hL);
+    // F+ - F-: mass, outward momentum, tangential momentum
+    const double gh = 0.5 * g * (hR - hL) * (hR + hL);
+    const double dFn = nR * uR - nL * uL + gh;
+    const double dFt = nR * vR - nL * vL;
+    double dN;
+    if (FK == DRF_FLUX_HLLC) {
+        const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
+        const double mL = hL * (SL - uL), mR = hR * (SR - uR), den = mL - mR;
+        const double Ss = fabs(den) > 1e-10 ? (uL * mL - uR * mR + gh) / den : 0.5 * (uL + uR);
+        if (SL >= 0) {
+            d[0] = dN = d[2] = 0.0;
+        } else if (SR <= 0) {
+            d[0] = dn; dN = dFn; d[2] = dFt;
+        } else {
+            const bool left = Ss >= 0;
+            const double S = left ? SL : SR, hs = (left ? mL : mR) / (S - Ss);
+            const double *K = left ? L : R;
+            d[0] = S * (hs - wet(K[0]));
+            dN = S * (hs * Ss - (left ? nL : nR));
+            d[2] = S * (hs * (left ? vL : vR) - K[2]);
+            if (!left) { d[0] += dn; dN += dFn; d[2] += dFt; }
+        }
+    } else {
+        const double sL = sqrt(hL), sR = sqrt(hR), is = 1.0 / (sL + sR);
+        const double hr = 0.5 * (hL + hR), ur = (sL * uL + sR * uR) * is, vr = (sL * vL + sR * vR) * is;
+        const double cr = sqrt(g * hr), delta = 0.1 * cr;
+        double l1 = fabs(ur - cr), l3 = fabs(ur + cr);
+        if (l1 < delta) l1 = (l1 * l1 + delta * delta) / (2.0 * delta);
+        if (l3 < delta) l3 = (l3 * l3 + delta * delta) / (2.0 * delta);
+        const double hh = hR - hL, q = hr / cr * (uR - uL);
+        const double a1 = l1 * 0.5 * (hh - q), a2 = fabs(ur) * (hr * (vR - vL)), a3 = l3 * 0.5 * (hh + q);
+        d[0] = 0.5 * (dn - (a1 + a3));
+        dN = 0.5 * (dFn - (a1 * (ur - cr) + a3 * (ur + cr)));
+        d[2] = 0.5 * (dFt - ((a1 + a3) * vr + a2));
+    }
+    d[1] = sg * dN;
 }
 
 // Register budget of the subcycle kernels: 800 resident threads per SM (80 registers) for up to
@@ -1222,73 +1276,54 @@ constexpr int baro_min_blocks(int threads, int np) {
 //    the element's threads (one flux per thread for N >= 3), not evaluated by the face nodes
 //    themselves, so no warp runs the flux twice (x then y) under divergence. Each item writes
 //    F*(U-, U+) - F(U-) to shared memory; a node subtracts its x face's, then its y face's.
-//  * Every global load (own state, the face items' neighbour values) is issued before the
-//    first tile barrier; the tidal elevation is evaluated only by items on a tidal side.
-template <int NP, int FK, int CPB>
-__device__ __forceinline__ bool baro_tile_phi(const BaroArgs &a, int64_t tile, double toff, double &re, double &ru,
-                                              double &rv, int64_t &t) {
-    constexpr int NP2 = NP * NP, N = NP - 1, NF = 4 * NP;
-    constexpr int NI = (NF + NP2 - 1) / NP2;  // face items per thread
-    __shared__ double sE[CPB * NP2], sU[CPB * NP2], sV[CPB * NP2], sB[CPB * NP2], sI[CPB * NP2];
-    __shared__ double sUU[CPB * NP2], sUV[CPB * NP2], sVV[CPB * NP2], sD[NP2];
-    __shared__ double sF[CPB * NF * 3];  // per element and face item: d = F* - F(U-)
-    const Geo &G = a.G;
+template <int NP, int CPB>
+struct BaroTile {
+    static constexpr int NP2 = NP * NP, NF = 4 * NP, NI = (NF + NP2 - 1) / NP2;  // NI: face items per thread
+    double E[CPB * NP2], U[CPB * NP2], V[CPB * NP2], B[CPB * NP2], I[CPB * NP2];
+    double UU[CPB * NP2], UV[CPB * NP2], VV[CPB * NP2], D[NP2];
+    double F[CPB * NF * 3];  // per element and face item: d = F* - F(U-)
+};
+
+// Phi without its forcing and faces at this thread's node (re, ru, rv), the faces' differences in
+// T.F. across(r, UR) gives the state (H, hu, hv) across this thread's face item r, or returns
+// false on a basin side; it is called after the tile's state is in shared memory. Two block barriers; with CANFAIL, false when
+// `fail` is set by any thread.
+template <int NP, int FK, bool CANFAIL, int CPB, class Across>
+__device__ __forceinline__ bool baro_tile_core(BaroTile<NP, CPB> &T, const Geo &G, bool valid, double e, double hu0,
+                                               double hv0, double hb, double fc, const double *tdev, double toff,
+                                               bool fail, Across &&across, double &re, double &ru, double &rv) {
+    using Tl = BaroTile<NP, CPB>;
+    constexpr int NP2 = NP * NP, N = NP - 1, NF = Tl::NF;
     const int lc = threadIdx.x / NP2, an = threadIdx.x % NP2, i = an % NP, j = an / NP;
-    const int64_t c = tile * CPB + lc;
-    const bool valid = c < a.ncol;
-    if (threadIdx.x < NP2) sD[threadIdx.x] = cBs[NP].D[threadIdx.x];
-    t = c * NP2 + an;
-    const int ex = (int)(c % G.nx), ey = (int)(c / G.nx);
-    double e = 0.0, hb = 0.0, hu0 = 0.0, hv0 = 0.0, fc = 0.0, fx = 0.0, fy = 0.0;
-    if (valid) {
-        e = a.e[t]; hb = a.h[t]; hu0 = a.hu[t]; hv0 = a.hv[t]; fc = a.f[t];
-        if (a.Fx) { fx = a.Fx[t]; fy = a.Fy[t]; }
-    }
-    // this thread's face items: side s = it / NP (0 -x, 1 +x, 2 -y, 3 +y), position k = it % NP;
-    // the neighbour's e, h, hu, hv across the face (q < 0 on a basin side)
-    int64_t qn[NI];
-    double nb[NI][4];
-#pragma unroll
-    for (int r = 0; r < NI; ++r) {
-        const int it = an + r * NP2;
-        qn[r] = -1;
-        nb[r][0] = nb[r][1] = nb[r][2] = nb[r][3] = 0.0;
-        if (!valid || it >= NF) continue;
-        const int s = it / NP, k = it % NP;
-        if (s == 0 && ex > 0) qn[r] = (c - 1) * NP2 + N + NP * k;
-        if (s == 1 && ex < G.nx - 1) qn[r] = (c + 1) * NP2 + NP * k;
-        if (s == 2 && ey > 0) qn[r] = (c - G.nx) * NP2 + k + NP * N;
-        if (s == 3 && ey < G.ny - 1) qn[r] = (c + G.nx) * NP2 + k;
-        if (qn[r] >= 0) {
-            nb[r][0] = a.e[qn[r]]; nb[r][1] = a.h[qn[r]]; nb[r][2] = a.hu[qn[r]]; nb[r][3] = a.hv[qn[r]];
-        }
-    }
     const double H = valid ? e + hb : 1.0;
     const double iH = 1.0 / H;
     if (valid) {
         const int n = threadIdx.x;
         const double u = hu0 * iH, v = hv0 * iH;
-        sE[n] = e; sU[n] = hu0; sV[n] = hv0; sB[n] = hb; sI[n] = iH;
-        sUU[n] = hu0 * u; sUV[n] = hv0 * u; sVV[n] = hv0 * v;
+        T.E[n] = e; T.U[n] = hu0; T.V[n] = hv0; T.B[n] = hb; T.I[n] = iH;
+        T.UU[n] = hu0 * u; T.UV[n] = hv0 * u; T.VV[n] = hv0 * v;
     }
-    __syncthreads();
+    if constexpr (CANFAIL) {
+        if (__syncthreads_or(fail)) return false;
+    } else {
+        __syncthreads();
+    }
     // face items: the flux difference at face node (fi, fj) of this element
 #pragma unroll
-    for (int r = 0; r < NI; ++r) {
+    for (int r = 0; r < Tl::NI; ++r) {
         const int it = an + r * NP2;
         if (!valid || it >= NF) continue;
         const int s = it / NP, k = it % NP;
         const int fi = s == 0 ? 0 : (s == 1 ? N : k), fj = s <= 1 ? k : (s == 2 ? 0 : N);
         const int ln = lc * NP2 + fi + NP * fj;
-        const double HL = sE[ln] + sB[ln];  // the node's own H, recomputed exactly
-        const double UL[3] = {HL, sU[ln], sV[ln]};
+        const double HL = T.E[ln] + T.B[ln];  // the node's own H, recomputed exactly
+        const double UL[3] = {HL, T.U[ln], T.V[ln]};
         const double nx = s == 0 ? -1.0 : (s == 1 ? 1.0 : 0.0);
         const double ny = s == 2 ? -1.0 : (s == 3 ? 1.0 : 0.0);
         double UR[3];
-        if (qn[r] >= 0) {
-            UR[0] = nb[r][0] + nb[r][1]; UR[1] = nb[r][2]; UR[2] = nb[r][3];
+        if (across(r, UR)) {
         } else if ((s == 0 ? G.bc[0] : (s == 1 ? G.bc[1] : (s == 2 ? G.bc[2] : G.bc[3]))) == DRF_BC_TIDE) {
-            UR[0] = tide_at(G, a.tdev[0] + toff) + sB[ln];
+            UR[0] = tide_at(G, tdev[0] + toff) + T.B[ln];
             const double rr = UR[0] / HL;
             UR[1] = UL[1] * rr; UR[2] = UL[2] * rr;
         } else {
@@ -1297,14 +1332,17 @@ __device__ __forceinline__ bool baro_tile_phi(const BaroArgs &a, int64_t tile, d
         }
         double d[3];
         if (FK == DRF_FLUX_LF) {
-            lf_minus_phys(UL, sI[ln], sqrt(G.g * (HL < 1e-10 ? 1e-10 : HL)), UR, nx, ny, G.g, d);
+            lf_minus_phys(UL, T.I[ln], sqrt(G.g * (HL < 1e-10 ? 1e-10 : HL)), UR, nx, ny, G.g, d);
         } else {
-            double Fs[3], Fm[3];
-            sw_flux(FK, UL, UR, nx, ny, G.g, Fs);
-            sw_phys_flux(UL, nx, ny, G.g, Fm);
-            d[0] = Fs[0] - Fm[0]; d[1] = Fs[1] - Fm[1]; d[2] = Fs[2] - Fm[2];
+            // in the face's components: along the axis, then across it
+            const bool ax = s <= 1;
+            const double L[3] = {HL, ax ? UL[1] : UL[2], ax ? UL[2] : UL[1]};
+            const double R[3] = {UR[0], ax ? UR[1] : UR[2], ax ? UR[2] : UR[1]};
+            double q[3];
+            axis_flux_diff<FK>(L, HL < 1e-10 ? 1e10 : T.I[ln], R, (s & 1) ? 1.0 : -1.0, G.g, q);
+            d[0] = q[0]; d[1] = ax ? q[1] : q[2]; d[2] = ax ? q[2] : q[1];
         }
-        double *o = sF + (lc * NF + it) * 3;
+        double *o = T.F + (lc * NF + it) * 3;
         o[0] = d[0]; o[1] = d[1]; o[2] = d[2];
     }
     const int b0 = lc * NP2;
@@ -1312,30 +1350,98 @@ __device__ __forceinline__ bool baro_tile_phi(const BaroArgs &a, int64_t tile, d
 #pragma unroll
     for (int m = 0; m < NP; ++m) {
         const int px = b0 + m + NP * j, py = b0 + i + NP * m;
-        const double dxm = sD[i * NP + m], dym = sD[j * NP + m];
-        dhu += dxm * sU[px];
-        dhv += dym * sV[py];
-        auu += dxm * sUU[px];
-        avu += dxm * sUV[px];
-        auv += dym * sUV[py];
-        avv += dym * sVV[py];
-        gex += dxm * sE[px];
-        gey += dym * sE[py];
+        const double dxm = T.D[i * NP + m], dym = T.D[j * NP + m];
+        dhu += dxm * T.U[px];
+        dhv += dym * T.V[py];
+        auu += dxm * T.UU[px];
+        avu += dxm * T.UV[px];
+        auv += dym * T.UV[py];
+        avv += dym * T.VV[py];
+        gex += dxm * T.E[px];
+        gey += dym * T.E[py];
     }
-    __syncthreads();  // the face items are in sF
-    if (!valid) return false;
+    __syncthreads();  // the face items are in T.F
+    if (!valid) return true;
     re = -(G.cx * dhu + G.cy * dhv);
-    ru = -(G.cx * auu + G.cy * auv) - G.g * H * G.cx * gex + fc * hv0 + fx;
-    rv = -(G.cx * avu + G.cy * avv) - G.g * H * G.cy * gey - fc * hu0 + fy;
-    // x face first, then y face (a corner node has both)
+    ru = -(G.cx * auu + G.cy * auv) - G.g * H * G.cx * gex + fc * hv0;
+    rv = -(G.cx * avu + G.cy * avv) - G.g * H * G.cy * gey - fc * hu0;
+    return true;
+}
+// adds the forcing, then the x face, then the y face (a corner node has both)
+template <int NP, int CPB>
+__device__ __forceinline__ void baro_tile_finish(const BaroTile<NP, CPB> &T, const Geo &G, double fx, double fy,
+                                                 double &re, double &ru, double &rv) {
+    constexpr int NP2 = NP * NP, N = NP - 1, NF = 4 * NP;
+    const int lc = threadIdx.x / NP2, an = threadIdx.x % NP2, i = an % NP, j = an / NP;
+    ru += fx;
+    rv += fy;
     if (i == 0 || i == N) {
-        const double *d = sF + (lc * NF + (i == 0 ? 0 : NP) + j) * 3;
+        const double *d = T.F + (lc * NF + (i == 0 ? 0 : NP) + j) * 3;
         re -= G.Lx * d[0]; ru -= G.Lx * d[1]; rv -= G.Lx * d[2];
     }
     if (j == 0 || j == N) {
-        const double *d = sF + (lc * NF + (j == 0 ? 2 * NP : 3 * NP) + i) * 3;
+        const double *d = T.F + (lc * NF + (j == 0 ? 2 * NP : 3 * NP) + i) * 3;
         re -= G.Ly * d[0]; ru -= G.Ly * d[1]; rv -= G.Ly * d[2];
     }
+}
+// the column across side s of column c (-1 on a basin side) and its node of position k
+template <int NP>
+__device__ __forceinline__ int64_t baro_across(const Geo &G, int64_t c, int ex, int ey, int s, int k, int &node) {
+    constexpr int N = NP - 1;
+    if (s == 0 && ex > 0) { node = N + NP * k; return c - 1; }
+    if (s == 1 && ex < G.nx - 1) { node = NP * k; return c + 1; }
+    if (s == 2 && ey > 0) { node = k + NP * N; return c - G.nx; }
+    if (s == 3 && ey < G.ny - 1) { node = k; return c + G.nx; }
+    return -1;
+}
+
+// Phi with its forcing at this thread's node from the global state; every global load (own state,
+// the face items' neighbour values) is issued before the first tile barrier.
+template <int NP, int FK, int CPB>
+__device__ __forceinline__ bool baro_tile_phi(const BaroArgs &a, int64_t tile, double toff, double &re, double &ru,
+                                              double &rv, int64_t &t) {
+    using Tl = BaroTile<NP, CPB>;
+    constexpr int NP2 = NP * NP;
+    __shared__ Tl T;
+    const Geo &G = a.G;
+    const int lc = threadIdx.x / NP2, an = threadIdx.x % NP2;
+    const int64_t c = tile * CPB + lc;
+    const bool valid = c < a.ncol;
+    if (threadIdx.x < NP2) T.D[threadIdx.x] = cBs[NP].D[threadIdx.x];
+    t = c * NP2 + an;
+    const int ex = (int)(c % G.nx), ey = (int)(c / G.nx);
+    double e = 0.0, hb = 0.0, hu0 = 0.0, hv0 = 0.0, fc = 0.0, fx = 0.0, fy = 0.0;
+    if (valid) {
+        e = a.e[t]; hb = a.h[t]; hu0 = a.hu[t]; hv0 = a.hv[t]; fc = a.f[t];
+        if (a.Fx) { fx = a.Fx[t]; fy = a.Fy[t]; }
+    }
+    // this thread's face items: side s = it / NP (0 -x, 1 +x, 2 -y, 3 +y), position k = it % NP;
+    // the neighbour's e, h, hu, hv across the face
+    bool has[Tl::NI];
+    double nb[Tl::NI][4];
+#pragma unroll
+    for (int r = 0; r < Tl::NI; ++r) {
+        const int it = an + r * NP2;
+        has[r] = false;
+        nb[r][0] = nb[r][1] = nb[r][2] = nb[r][3] = 0.0;
+        if (!valid || it >= Tl::NF) continue;
+        int node = 0;
+        const int64_t nc = baro_across<NP>(G, c, ex, ey, it / NP, it % NP, node);
+        if (nc < 0) continue;
+        const int64_t q = nc * NP2 + node;
+        has[r] = true;
+        nb[r][0] = a.e[q]; nb[r][1] = a.h[q]; nb[r][2] = a.hu[q]; nb[r][3] = a.hv[q];
+    }
+    baro_tile_core<NP, FK, false>(
+        T, G, valid, e, hu0, hv0, hb, fc, a.tdev, toff, false,
+        [&](int r, double *q) {
+            if (!has[r]) return false;
+            q[0] = nb[r][0] + nb[r][1]; q[1] = nb[r][2]; q[2] = nb[r][3];
+            return true;
+        },
+        re, ru, rv);
+    if (!valid) return false;
+    baro_tile_finish<NP, CPB>(T, G, fx, fy, re, ru, rv);
     return true;
 }
 
@@ -1705,6 +1811,242 @@ __global__ void BARO_BOUNDS baro_subcycles_kernel(const __grid_constant__ BaroAr
     }
 }
 
+// ------------------------------------------------------- resident barotropic step (FP64)
+// The nsub Heun subcycles and the finish pass, after the forcing pass, for a model whose 2D nodes
+// fit on the chip one per thread: every CTA keeps its tile's state in registers and shared memory
+// through all of them, and meets only the tiles across its faces, without a grid-wide barrier. After
+// a pass a node on a tile's outer face publishes (e, hu, hv) in its trace slot, each value in
+// one 16-byte word with the pass's sequence number; the face item that needs it polls that word.
+// One store and one load cross the chip per pass. Predictor and corrector traces alternate
+// between two buffers: a tile writes a buffer again two passes later, after it has read its
+// neighbours' traces of the pass between, which they publish after reading this buffer.
+// Sequence numbers grow from launch to launch (the epoch word), so no trace is taken for
+// another step's. The launch is cooperative (all CTAs resident) and every poll is bounded.
+//
+// Bound by latency: an exchange and the dependent chain of a face flux (a reciprocal, a square
+// root) per pass, 1.5 us at C1 (256 columns, N = 3) against 3.3 us for a launch per pass.
+struct ResidentArgs {
+    double dt, dtb;
+    int nsub, ncol;
+    const double *h, *f, *Fx, *Fy, *dHU3, *dHV3, *etbf;
+    double *eta, *HU, *HV, *eta_avg, *corrU, *corrV, *corrR, *tdev;
+    ulonglong2 *trace;  // [2][column][side][face node][e, hu, hv]: value, sequence number
+    unsigned *sync;     // [0] epoch, [1] CTAs finished, [2] abort; the last CTA leaves [1], [2] zero
+    int *err;
+    int hold;  // failure-detection check: this CTA publishes no trace (-1: none)
+    Geo G;
+};
+__device__ __forceinline__ void trace_put(ulonglong2 *p, double v, uint64_t seq) {
+    uint64_t g;
+    asm volatile("cvta.to.global.u64 %0, %1;" : "=l"(g) : "l"(p));
+    asm volatile("{ .reg .b128 q; mov.b128 q, {%1, %2}; st.relaxed.gpu.global.b128 [%0], q; }" ::"l"(g),
+                 "l"(__double_as_longlong(v)), "l"(seq)
+                 : "memory");
+}
+__device__ __forceinline__ double trace_get(const ulonglong2 *p, uint64_t &seq) {
+    uint64_t g, v;
+    asm volatile("cvta.to.global.u64 %0, %1;" : "=l"(g) : "l"(p));
+    asm volatile("{ .reg .b128 q; ld.relaxed.gpu.global.b128 q, [%2]; mov.b128 {%0, %1}, q; }"
+                 : "=l"(v), "=l"(seq)
+                 : "l"(g)
+                 : "memory");
+    return __longlong_as_double(v);
+}
+
+// Columns per CTA: the smallest tile of at least 32 threads (C1's 2 columns against 4 and 8: 121, 123
+// and 132 us a step; 96 x 96 columns at N = 1, 8 against 2: 388 and 461 us).
+template <int NP>
+constexpr int resident_cpb() {
+    return NP == 2 ? 8 : (NP == 3 ? 4 : 2);
+}
+// CTAs per SM: 512 threads (128 registers, no spills) for the models that fit so, 896 (72
+// registers, spills at most orders; 640 at 6 x 6 nodes) for those that only fit then. The wide form
+// costs C1 129 instead of 121 us a step, and lets 64 x 64 columns at N = 4 take the resident
+// form: 268 us of barotropic work a step in 42 launches, 178 us resident.
+template <int NP>
+constexpr int resident_ctas(bool wide) {
+    const int t = (resident_cpb<NP>() * NP * NP + 31) / 32 * 32;
+    return (wide ? (NP <= 5 ? 896 : 640) : 512) / t;
+}
+
+template <int NP, int FK, bool WIDE>
+__global__ void __launch_bounds__(resident_cpb<NP>() * NP * NP, resident_ctas<NP>(WIDE))
+    baro_resident_kernel(const __grid_constant__ ResidentArgs a) {
+    constexpr int CPB = resident_cpb<NP>();
+    using Tl = BaroTile<NP, CPB>;
+    constexpr int NP2 = NP * NP, N = NP - 1;
+    constexpr int NT = CPB * NP2;
+    __shared__ Tl T;
+    // what a node keeps between passes: U^m, k1, the forcing and eta's sum (this thread's own
+    // entries, out of the registers the flux needs)
+    __shared__ double sE[NT], sU[NT], sV[NT], sKe[NT], sKu[NT], sKv[NT], sFx[NT], sFy[NT], sSum[NT];
+    const Geo &G = a.G;
+    const int me = threadIdx.x;
+    const int lc = threadIdx.x / NP2, an = threadIdx.x % NP2, i = an % NP, j = an / NP;
+    const int tile = blockIdx.x, c = tile * CPB + lc;
+    const bool valid = c < a.ncol;
+    if (threadIdx.x < NP2) T.D[threadIdx.x] = cBs[NP].D[threadIdx.x];
+    const uint64_t seq0 = ((uint64_t) * (volatile unsigned *)&a.sync[0] + 1) << 20;
+    const size_t t = (size_t)c * NP2 + an;
+    const int ex = c % G.nx, ey = c / G.nx;
+    double hb = 0.0, fc = 0.0, xe = 0.0, xu = 0.0, xv = 0.0;  // x: the state Phi is evaluated at
+    if (valid) {
+        xe = sE[me] = a.eta[t];
+        xu = sU[me] = a.HU[t];
+        xv = sV[me] = a.HV[t];
+        sFx[me] = a.Fx[t];
+        sFy[me] = a.Fy[t];
+        hb = a.h[t];
+        fc = a.f[t];
+    }
+    // face items: the neighbour's node in this tile (loc) or its trace slot (slot), -1 neither
+    int loc[Tl::NI], slot[Tl::NI];
+    double nb[Tl::NI][3], hbn[Tl::NI];
+#pragma unroll
+    for (int r = 0; r < Tl::NI; ++r) {
+        const int it = an + r * NP2, s = it / NP, k = it % NP;
+        loc[r] = slot[r] = -1;
+        hbn[r] = nb[r][0] = nb[r][1] = nb[r][2] = 0.0;
+        if (!valid || it >= Tl::NF) continue;
+        int node = 0;
+        const int nc = (int)baro_across<NP>(G, c, ex, ey, s, k, node);
+        if (nc < 0) continue;
+        if (nc / CPB == tile) {
+            loc[r] = (nc - tile * CPB) * NP2 + node;
+            continue;
+        }
+        slot[r] = (nc * 4 + (s ^ 1)) * NP + k;
+        const size_t q = (size_t)nc * NP2 + node;
+        hbn[r] = a.h[q];
+        nb[r][0] = a.eta[q]; nb[r][1] = a.HU[q]; nb[r][2] = a.HV[q];
+    }
+    // the trace slots this node publishes: its x face's and its y face's, across a tile boundary
+    auto outer = [&](int s) {
+        int node;
+        const int nc = valid ? (int)baro_across<NP>(G, c, ex, ey, s, 0, node) : -1;
+        return nc >= 0 && nc / CPB != tile && (int)blockIdx.x != a.hold;
+    };
+    const int px = i == 0 && outer(0) ? (c * 4 + 0) * NP + j : (i == N && outer(1) ? (c * 4 + 1) * NP + j : -1);
+    const int py = j == 0 && outer(2) ? (c * 4 + 2) * NP + i : (j == N && outer(3) ? (c * 4 + 3) * NP + i : -1);
+    const size_t half = (size_t)a.ncol * 4 * NP * 3;
+    const double hd = 0.5 * a.dtb;
+    bool ok = true;
+    for (int p = 0; p < 2 * a.nsub; ++p) {  // predictor (even p) and corrector passes
+        const double tm = __dmul_rn((double)(p >> 1), a.dtb);
+        bool fail = false;
+        if (p > 0) {  // the neighbours' traces of the pass before
+            const ulonglong2 *tr = a.trace + (size_t)(p & 1) * half;
+            const uint64_t want = seq0 + p;
+#pragma unroll
+            for (int r = 0; r < Tl::NI; ++r) {
+                if (slot[r] < 0) continue;
+                const ulonglong2 *w = tr + (size_t)slot[r] * 3;
+                for (int it = 0;; ++it) {
+                    uint64_t q0, q1, q2;
+                    nb[r][0] = trace_get(w, q0);
+                    nb[r][1] = trace_get(w + 1, q1);
+                    nb[r][2] = trace_get(w + 2, q2);
+                    if (q0 == want && q1 == want && q2 == want) break;
+                    if (it > (1 << 20) || ((it & 255) == 255 && *(volatile unsigned *)&a.sync[2] != 0u)) {
+                        fail = true;
+                        break;
+                    }
+                }
+            }
+        }
+        double re, ru, rv;
+        ok = baro_tile_core<NP, FK, true>(
+            T, G, valid, xe, xu, xv, hb, fc, a.tdev, (p & 1) ? __dadd_rn(tm, a.dtb) : tm, fail,
+            [&](int r, double *q) {
+                if (loc[r] >= 0) {
+                    q[0] = T.E[loc[r]] + T.B[loc[r]]; q[1] = T.U[loc[r]]; q[2] = T.V[loc[r]];
+                    return true;
+                }
+                if (slot[r] < 0) return false;
+                q[0] = nb[r][0] + hbn[r]; q[1] = nb[r][1]; q[2] = nb[r][2];
+                return true;
+            },
+            re, ru, rv);
+        if (!ok) break;
+        if (!valid) continue;
+        baro_tile_finish<NP, CPB>(T, G, sFx[me], sFy[me], re, ru, rv);
+        if (p & 1) {
+            sE[me] = xe = sE[me] + hd * (sKe[me] + re);
+            sU[me] = xu = sU[me] + hd * (sKu[me] + ru);
+            sV[me] = xv = sV[me] + hd * (sKv[me] + rv);
+            sSum[me] = (p == 1 ? 0.0 : sSum[me]) + xe;
+        } else {
+            sKe[me] = re; sKu[me] = ru; sKv[me] = rv;
+            xe = sE[me] + a.dtb * re; xu = sU[me] + a.dtb * ru; xv = sV[me] + a.dtb * rv;
+        }
+        if (p + 1 < 2 * a.nsub) {
+            ulonglong2 *tr = a.trace + (size_t)((p + 1) & 1) * half;
+            const uint64_t seq = seq0 + p + 1;
+            if (px >= 0) {
+                trace_put(tr + (size_t)px * 3, xe, seq);
+                trace_put(tr + (size_t)px * 3 + 1, xu, seq);
+                trace_put(tr + (size_t)px * 3 + 2, xv, seq);
+            }
+            if (py >= 0) {
+                trace_put(tr + (size_t)py * 3, xe, seq);
+                trace_put(tr + (size_t)py * 3 + 1, xu, seq);
+                trace_put(tr + (size_t)py * 3 + 2, xv, seq);
+            }
+        }
+    }
+    // the state, eta's time mean and the transport correction; the neighbours read U^n of this
+    // tile before they published the first trace this tile has waited for
+    if (ok && valid) {
+        const double uo = a.HU[t], vo = a.HV[t];
+        a.eta[t] = xe; a.HU[t] = xu; a.HV[t] = xv;
+        a.eta_avg[t] = sSum[me] / a.nsub;
+        a.corrU[t] = xu - (uo + a.dHU3[t]);
+        a.corrV[t] = xv - (vo + a.dHV3[t]);
+        a.corrR[t] = tracer_volume_correction(xe, a.etbf[t], hb);
+    }
+    if (!ok && threadIdx.x == 0) {
+        atomicExch(&a.sync[2], 1u);
+        atomicExch(a.err, DRF_E_TIMEOUT);
+    }
+    // the last CTA to finish: the clock advances once every CTA is past its last read of it
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&a.sync[1], 1u) == gridDim.x - 1) {
+            __threadfence();
+            a.sync[0] += 1;
+            a.sync[1] = 0;
+            if (atomicExch(&a.sync[2], 0u) == 0u) a.tdev[0] = a.tdev[0] + a.dt;
+        }
+    }
+}
+
+// water columns the resident form takes: those of the CTAs that can be on the chip together
+template <int NP, int FK, bool WIDE>
+int64_t resident_columns() {
+    constexpr int CPB = resident_cpb<NP>();
+    int dev = 0, nsm = 0, per_sm = 0;
+    DRF_CUDA(cudaGetDevice(&dev));
+    DRF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    DRF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, baro_resident_kernel<NP, FK, WIDE>, CPB * NP * NP, 0));
+    return (int64_t)per_sm * nsm * CPB;
+}
+template <int NP, int FK, bool WIDE>
+void launch_resident(const ResidentArgs &a, cudaStream_t st) {
+    constexpr int CPB = resident_cpb<NP>();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((a.ncol + CPB - 1) / CPB));
+    cfg.blockDim = dim3((unsigned)(CPB * NP * NP));
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    DRF_CUDA(cudaLaunchKernelEx(&cfg, baro_resident_kernel<NP, FK, WIDE>, a));
+    DRF_LAUNCHED();
+}
+
 // Launches baro_subcycles_kernel cooperatively, with as many CTAs as can be resident (at most
 // one per tile), after zeroing its barrier words on the same stream.
 template <int NP, int FK, int CPB, bool ENS>
@@ -1982,10 +2324,14 @@ struct drf_dg {
     // barotropic step as one persistent launch (false: one launch per pass); fixed when the
     // step graphs are built, from DRIFTER_B200_BARO_PERSISTENT (1 selects the persistent form)
     bool baro_persist = false;
-    // failure-detection check of the persistent barotropic launch: the CTA that withholds its
-    // first grid-barrier arrival (-1 none); fixed when the step graphs are built, from
-    // DRIFTER_B200_DEBUG_HOLD_ARRIVAL
+    // failure-detection check of the persistent and resident barotropic launches: the CTA that
+    // withholds its first grid-barrier arrival, or its traces (-1 none); fixed when the step
+    // graphs are built, from DRIFTER_B200_DEBUG_HOLD_ARRIVAL
     int debug_hold = -1;
+    // resident form of the barotropic step (resident_form; fixed when the step graphs are
+    // built) and its trace slots
+    int baro_res = 0;
+    DevBuf<ulonglong2> trace;
     // 3D arrays: q3p + (array * n3s + node) * tsz; n3s = n3 for a model that owns its memory,
     // the pool length for an ensemble member (a view into the ensemble's pools)
     unsigned char *q3p = nullptr;
@@ -2166,6 +2512,30 @@ struct drf_dg {
         return s;
     }
 
+    // Whether the barotropic step takes the resident form (0 no, 1 roomy, 2 wide): where the
+    // model fits it, as one launch then replaces 2 nsub + 1 and a pass costs one exchange of
+    // traces instead of a launch (per step, both measured: C1 198 -> 126 us, 23 x 17 columns at
+    // N = 2 with HLLC 280 -> 184 us, 64 x 64 at N = 4 1221 -> 1139 us). Launch forms fixed by
+    // DRIFTER_B200_TUNE=0 or DRIFTER_B200_BARO_PERSISTENT stay as they are.
+    int resident_form(int nsub) {
+        const char *tu = std::getenv("DRIFTER_B200_TUNE"), *pe = std::getenv("DRIFTER_B200_BARO_PERSISTENT");
+        // sequence numbers hold 2^20 passes a launch
+        if (view || (tu && tu[0] == '0') || (pe && pe[0]) || nsub >= (1 << 19)) return 0;
+        int form = 0;
+        dispatch_np(np, [&](auto npc) {
+            constexpr int NP = decltype(npc)::value;
+            dispatch_flux(G.flux2d, [&](auto fk) {
+                constexpr int FK = decltype(fk)::value;
+                form = ncol <= resident_columns<NP, FK, false>() ? 1 : (ncol <= resident_columns<NP, FK, true>() ? 2 : 0);
+            });
+        });
+        if (form && !trace.n) {
+            trace.alloc((size_t)2 * ncol * 4 * np * 3);
+            DRF_CUDA(cudaMemsetAsync(trace.p, 0, trace.n * sizeof(ulonglong2), stream));
+        }
+        return form;
+    }
+
     template <typename T, int NP>
     void enqueue_step(int in, double dt, int nsub) {
         const int out = 1 - in;
@@ -2177,6 +2547,29 @@ struct drf_dg {
             src = dst;
         }
         // after 5 stages the state is in `out`; the barotropic tile is the tuned one
+        if (baro_res) {
+            dispatch_cpb(baro_cpb, [&](auto cpbc) {
+                constexpr int CPB = decltype(cpbc)::value;
+                dispatch_flux(G.flux2d, [&](auto fk) {
+                    constexpr int FK = decltype(fk)::value;
+                    baro_force_kernel<NP, FK, CPB><<<(unsigned)((ncol + CPB - 1) / CPB), CPB * NP * NP, 0, stream>>>(
+                        baro<NP>(eta, HU, HV, false, 0.0), dt, dHU3, dHV3, Fx, Fy, HUo, HVo);
+                });
+            });
+            DRF_LAUNCHED();
+            ResidentArgs r{};
+            r.dt = dt; r.dtb = dt / nsub; r.nsub = nsub; r.ncol = ncol;
+            r.h = h; r.f = f; r.Fx = Fx; r.Fy = Fy; r.dHU3 = dHU3; r.dHV3 = dHV3; r.etbf = etb[0];
+            r.eta = eta; r.HU = HU; r.HV = HV; r.eta_avg = eta_avg;
+            r.corrU = corrU; r.corrV = corrV; r.corrR = corrR; r.tdev = tdev;
+            r.trace = trace.p; r.sync = syncbuf.p; r.err = err; r.hold = debug_hold; r.G = G;
+            dispatch_flux(G.flux2d, [&](auto fk) {
+                constexpr int FK = decltype(fk)::value;
+                if (baro_res == 1) launch_resident<NP, FK, false>(r, stream);
+                else launch_resident<NP, FK, true>(r, stream);
+            });
+            return;
+        }
         if (baro_persist) {
             dispatch_cpb(baro_cpb, [&](auto cpbc) {
                 constexpr int CPB = decltype(cpbc)::value;
@@ -2768,6 +3161,7 @@ int drf_dg_step_modesplit(drf_dg *m, double dt, int nsub, int nsteps) {
             m->baro_persist = pe && pe[0] == '1';
             const char *ph = std::getenv("DRIFTER_B200_DEBUG_HOLD_ARRIVAL");
             m->debug_hold = ph && ph[0] ? std::atoi(ph) : -1;
+            m->baro_res = m->resident_form(nsub);
             for (int in = 0; in < 2; ++in)
                 m->graph[in] = capture_graph(m->stream, [&] {
                     m->with_types([&](auto tv, auto npc) {

@@ -317,6 +317,98 @@ def test_persistent_barotropic_step_agrees_with_per_pass_launches(monkeypatch, p
         assert relerr(a[k], b[k]) <= 1e-11, (k, relerr(a[k], b[k]))
 
 
+def _step_pair(case, monkeypatch, steps=2):
+    """The same steps in the library's own form and with one launch per barotropic pass, with the
+    launches of each."""
+    out = []
+    for env in (None, "0"):
+        if env:
+            monkeypatch.setenv("DRIFTER_B200_BARO_PERSISTENT", env)
+        m = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+        m.upload_state(case["q"], case["eta"])
+        m.step(case["dt"], case["nsub"], 0)
+        before = launch_count()
+        m.step(case["dt"], case["nsub"], steps)
+        m.sync()
+        launched = launch_count() - before
+        out.append((m.download_state(), launched))
+        m.close()
+    monkeypatch.delenv("DRIFTER_B200_BARO_PERSISTENT")
+    return out
+
+
+# odd column counts leave the last tile part empty; 61 x 61 columns at N = 4 (93,025 nodes) take the
+# wide instance, 1 x 1 has no face across tiles
+@pytest.mark.parametrize("order,nx,ny,flux2d,nsub", [(1, 7, 5, "lf", 4), (2, 9, 7, "hllc", 3), (3, 5, 5, "roe", 20),
+                                                     (3, 1, 1, "lf", 2), (4, 11, 3, "lf", 1), (4, 61, 61, "lf", 3),
+                                                     (5, 3, 9, "hllc", 2)])
+def test_resident_barotropic_step_equals_per_pass_launches(monkeypatch, order, nx, ny, flux2d, nsub):
+    """A model whose 2D nodes fit on the chip takes the barotropic subcycles as one launch; each node
+    does the per-pass kernels' operations, so the two forms agree to the 1e-11 of the cooperative
+    form's test (the compiler may fuse a multiply-add differently)."""
+    case = _tidal_small("fp64", order=order, nx=nx, ny=ny, nz=1, flux2d=flux2d)
+    case["dt"] *= nsub / case["nsub"] * min(1.0, 5.0 / max(nx, ny))
+    case["nsub"] = nsub
+    (a, na), (b, nb) = _step_pair(case, monkeypatch)
+    assert na == 2 * 7 and nb == 2 * (5 + 2 + 2 * nsub)
+    assert a["t"] == b["t"] and np.abs(a["eta"]).max() < 10.0
+    for k in ("eta", "HU", "HV", "eta_avg", "Hu", "Hv", "HT", "HS"):
+        assert relerr(a[k], b[k]) <= 1e-11, (k, relerr(a[k], b[k]))
+
+
+def test_resident_barotropic_steps_of_two_models_at_once():
+    """Two models step on their own streams from two host threads, their resident launches in
+    flight together: each ends where it does alone."""
+    import threading
+    cases = [_tidal_small("fp64", nx=9, ny=7), _tidal_small("fp64", order=4, nx=8, ny=11)]
+
+    def run(case):
+        m = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+        m.upload_state(case["q"], case["eta"])
+        for _ in range(20):
+            m.step(case["dt"], case["nsub"], 1)
+        s = m.download_state()
+        m.close()
+        return s
+
+    alone = [run(c) for c in cases]
+    got = [None, None]
+
+    def work(i):
+        got[i] = run(cases[i])
+
+    th = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for a, g in zip(alone, got):
+        for k in ("eta", "HU", "HV", "Hu", "HT"):
+            assert relerr(g[k], a[k]) == 0.0, k
+
+
+def test_bounded_trace_wait_gives_up_and_the_model_stays_usable(monkeypatch):
+    """Failure detection of the resident form without a GPU fault: with
+    DRIFTER_B200_DEBUG_HOLD_ARRIVAL=0 its CTA 0 publishes no trace, so the bounded polls of the
+    tiles across its faces give up, the launch ends with the status word set and the host reads
+    DRF_E_TIMEOUT. The next step of a model built afterwards agrees with the per-pass form."""
+    from drifter_b200 import DrfError
+    case = _tidal_small("fp64", nx=9, ny=7)
+    monkeypatch.setenv("DRIFTER_B200_DEBUG_HOLD_ARRIVAL", "0")
+    held = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+    held.upload_state(case["q"], case["eta"])
+    held.step(case["dt"], case["nsub"], 1)
+    with pytest.raises(DrfError) as ei:
+        held.sync()
+    assert ei.value.code == 6  # DRF_E_TIMEOUT
+    held.sync()  # the status word was cleared
+    held.close()
+    monkeypatch.delenv("DRIFTER_B200_DEBUG_HOLD_ARRIVAL")
+    (a, _), (b, _) = _step_pair(case, monkeypatch)
+    for k in ("eta", "HU", "Hu", "HT"):
+        assert relerr(a[k], b[k]) <= 1e-11, k
+
+
 def test_bounded_grid_barrier_wait_gives_up_and_the_model_stays_usable(monkeypatch):
     """Failure detection without a GPU fault. With DRIFTER_B200_DEBUG_HOLD_ARRIVAL=0 the
     persistent barotropic launch's CTA 0 withholds its arrival at the first grid barrier, so no
