@@ -1207,15 +1207,15 @@ __device__ __forceinline__ void lf_minus_phys(const double UL[3], double ihL, do
     }
 }
 
-// d = F*(U-, U+, n) - F(U-).n for a face normal along an axis, in the face's own components:
+// d = F*(U-, U+, n) - F(U-).n of the HLLC flux for a face normal along an axis, in the face's own components:
 // U = (h, hn, ht) with hn, ht the momentum along and across the axis, sg = +-1 the outward
 // direction along it, iL = 1 / h- (clamped as below). The interior flux is taken out of F*
 // algebraically, which also takes out the cancellation of their 0.5 g h^2. Same states, speeds and
-// branches as sw_flux; one division per state and speed instead of seven and more (23 x 17 columns at
-// N = 2 with HLLC, resident form: 178 us a step against 208 us with F* and F- formed separately).
+// branches as sw_flux; one division per state and speed instead of seven and more. For the resident
+// form, whose passes wait for the longest chain (23 x 17 columns at N = 2: 184 us a step against
+// 208 us with F* and F- formed separately); a launch per pass gains 2%, and keeps sw_flux.
 __device__ __forceinline__ double wet(double h) { return h < 1e-10 ? 1e-10 : h; }
-template <int FK>
-__device__ __forceinline__ void axis_flux_diff(const double L[3], double iL, const double R[3], double sg, double g,
+__device__ __forceinline__ void hllc_flux_diff(const double L[3], double iL, const double R[3], double sg, double g,
                                                double d[3]) {
     const double hL = wet(L[0]), hR = wet(R[0]), iR = 1.0 / hR;
     const double nL = sg * L[1], nR = sg * R[1];  // outward momenta
@@ -1228,35 +1228,21 @@ __device__ __forceinline__ void axis_flux_diff(const double L[3], double iL, con
     const double dFn = nR * uR - nL * uL + gh;
     const double dFt = nR * vR - nL * vL;
     double dN;
-    if (FK == DRF_FLUX_HLLC) {
-        const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
-        const double mL = hL * (SL - uL), mR = hR * (SR - uR), den = mL - mR;
-        const double Ss = fabs(den) > 1e-10 ? (uL * mL - uR * mR + gh) / den : 0.5 * (uL + uR);
-        if (SL >= 0) {
-            d[0] = dN = d[2] = 0.0;
-        } else if (SR <= 0) {
-            d[0] = dn; dN = dFn; d[2] = dFt;
-        } else {
-            const bool left = Ss >= 0;
-            const double S = left ? SL : SR, hs = (left ? mL : mR) / (S - Ss);
-            const double *K = left ? L : R;
-            d[0] = S * (hs - wet(K[0]));
-            dN = S * (hs * Ss - (left ? nL : nR));
-            d[2] = S * (hs * (left ? vL : vR) - K[2]);
-            if (!left) { d[0] += dn; dN += dFn; d[2] += dFt; }
-        }
+    const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
+    const double mL = hL * (SL - uL), mR = hR * (SR - uR), den = mL - mR;
+    const double Ss = fabs(den) > 1e-10 ? (uL * mL - uR * mR + gh) / den : 0.5 * (uL + uR);
+    if (SL >= 0) {
+        d[0] = dN = d[2] = 0.0;
+    } else if (SR <= 0) {
+        d[0] = dn; dN = dFn; d[2] = dFt;
     } else {
-        const double sL = sqrt(hL), sR = sqrt(hR), is = 1.0 / (sL + sR);
-        const double hr = 0.5 * (hL + hR), ur = (sL * uL + sR * uR) * is, vr = (sL * vL + sR * vR) * is;
-        const double cr = sqrt(g * hr), delta = 0.1 * cr;
-        double l1 = fabs(ur - cr), l3 = fabs(ur + cr);
-        if (l1 < delta) l1 = (l1 * l1 + delta * delta) / (2.0 * delta);
-        if (l3 < delta) l3 = (l3 * l3 + delta * delta) / (2.0 * delta);
-        const double hh = hR - hL, q = hr / cr * (uR - uL);
-        const double a1 = l1 * 0.5 * (hh - q), a2 = fabs(ur) * (hr * (vR - vL)), a3 = l3 * 0.5 * (hh + q);
-        d[0] = 0.5 * (dn - (a1 + a3));
-        dN = 0.5 * (dFn - (a1 * (ur - cr) + a3 * (ur + cr)));
-        d[2] = 0.5 * (dFt - ((a1 + a3) * vr + a2));
+        const bool left = Ss >= 0;
+        const double S = left ? SL : SR, hs = (left ? mL : mR) / (S - Ss);
+        const double *K = left ? L : R;
+        d[0] = S * (hs - wet(K[0]));
+        dN = S * (hs * Ss - (left ? nL : nR));
+        d[2] = S * (hs * (left ? vL : vR) - K[2]);
+        if (!left) { d[0] += dn; dN += dFn; d[2] += dFt; }
     }
     d[1] = sg * dN;
 }
@@ -1286,9 +1272,9 @@ struct BaroTile {
 
 // Phi without its forcing and faces at this thread's node (re, ru, rv), the faces' differences in
 // T.F. across(r, UR) gives the state (H, hu, hv) across this thread's face item r, or returns
-// false on a basin side; it is called after the tile's state is in shared memory. Two block barriers; with CANFAIL, false when
+// false on a basin side; it is called after the tile's state is in shared memory. Two block barriers; in the resident form, false when
 // `fail` is set by any thread.
-template <int NP, int FK, bool CANFAIL, int CPB, class Across>
+template <int NP, int FK, bool RESIDENT, int CPB, class Across>
 __device__ __forceinline__ bool baro_tile_core(BaroTile<NP, CPB> &T, const Geo &G, bool valid, double e, double hu0,
                                                double hv0, double hb, double fc, const double *tdev, double toff,
                                                bool fail, Across &&across, double &re, double &ru, double &rv) {
@@ -1303,7 +1289,7 @@ __device__ __forceinline__ bool baro_tile_core(BaroTile<NP, CPB> &T, const Geo &
         T.E[n] = e; T.U[n] = hu0; T.V[n] = hv0; T.B[n] = hb; T.I[n] = iH;
         T.UU[n] = hu0 * u; T.UV[n] = hv0 * u; T.VV[n] = hv0 * v;
     }
-    if constexpr (CANFAIL) {
+    if constexpr (RESIDENT) {
         if (__syncthreads_or(fail)) return false;
     } else {
         __syncthreads();
@@ -1331,7 +1317,12 @@ __device__ __forceinline__ bool baro_tile_core(BaroTile<NP, CPB> &T, const Geo &
             if (s <= 1) UR[1] = -UL[1]; else UR[2] = -UL[2];
         }
         double d[3];
-        if (FK == DRF_FLUX_LF) {
+        if (FK == DRF_FLUX_ROE || (FK == DRF_FLUX_HLLC && !RESIDENT)) {
+            double Fs[3], Fm[3];
+            sw_flux(FK, UL, UR, nx, ny, G.g, Fs);
+            sw_phys_flux(UL, nx, ny, G.g, Fm);
+            d[0] = Fs[0] - Fm[0]; d[1] = Fs[1] - Fm[1]; d[2] = Fs[2] - Fm[2];
+        } else if (FK == DRF_FLUX_LF) {
             lf_minus_phys(UL, T.I[ln], sqrt(G.g * (HL < 1e-10 ? 1e-10 : HL)), UR, nx, ny, G.g, d);
         } else {
             // in the face's components: along the axis, then across it
@@ -1339,7 +1330,7 @@ __device__ __forceinline__ bool baro_tile_core(BaroTile<NP, CPB> &T, const Geo &
             const double L[3] = {HL, ax ? UL[1] : UL[2], ax ? UL[2] : UL[1]};
             const double R[3] = {UR[0], ax ? UR[1] : UR[2], ax ? UR[2] : UR[1]};
             double q[3];
-            axis_flux_diff<FK>(L, HL < 1e-10 ? 1e10 : T.I[ln], R, (s & 1) ? 1.0 : -1.0, G.g, q);
+            hllc_flux_diff(L, HL < 1e-10 ? 1e10 : T.I[ln], R, (s & 1) ? 1.0 : -1.0, G.g, q);
             d[0] = q[0]; d[1] = ax ? q[1] : q[2]; d[2] = ax ? q[2] : q[1];
         }
         double *o = T.F + (lc * NF + it) * 3;
@@ -1395,6 +1386,27 @@ __device__ __forceinline__ int64_t baro_across(const Geo &G, int64_t c, int ex, 
     return -1;
 }
 
+// The subcycle launches overlap: each lets the next one's CTAs start as its own last wave runs
+// (launch_dependents at its start), and waits for the launch before it only at its first read of
+// what that one writes. C2: 767 us of barotropic work
+// a step, 741 us with it; 24 members of 16 to 40 columns a side 1731 and 1678 us a step.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+void launch_overlapped(void (*kern)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    DRF_CUDA(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+    DRF_LAUNCHED();
+}
+
 // Phi with its forcing at this thread's node from the global state; every global load (own state,
 // the face items' neighbour values) is issued before the first tile barrier.
 template <int NP, int FK, int CPB>
@@ -1411,31 +1423,38 @@ __device__ __forceinline__ bool baro_tile_phi(const BaroArgs &a, int64_t tile, d
     t = c * NP2 + an;
     const int ex = (int)(c % G.nx), ey = (int)(c / G.nx);
     double e = 0.0, hb = 0.0, hu0 = 0.0, hv0 = 0.0, fc = 0.0, fx = 0.0, fy = 0.0;
-    if (valid) {
-        e = a.e[t]; hb = a.h[t]; hu0 = a.hu[t]; hv0 = a.hv[t]; fc = a.f[t];
-        if (a.Fx) { fx = a.Fx[t]; fy = a.Fy[t]; }
-    }
     // this thread's face items: side s = it / NP (0 -x, 1 +x, 2 -y, 3 +y), position k = it % NP;
-    // the neighbour's e, h, hu, hv across the face
-    bool has[Tl::NI];
+    // the neighbour's e, h, hu, hv across the face (its node, -1 on a basin side)
+    int64_t qn[Tl::NI];
     double nb[Tl::NI][4];
+    // what no earlier launch writes is loaded while the launch before may still run
+    if (valid) { hb = a.h[t]; fc = a.f[t]; }
 #pragma unroll
     for (int r = 0; r < Tl::NI; ++r) {
         const int it = an + r * NP2;
-        has[r] = false;
+        qn[r] = -1;
         nb[r][0] = nb[r][1] = nb[r][2] = nb[r][3] = 0.0;
         if (!valid || it >= Tl::NF) continue;
         int node = 0;
         const int64_t nc = baro_across<NP>(G, c, ex, ey, it / NP, it % NP, node);
         if (nc < 0) continue;
-        const int64_t q = nc * NP2 + node;
-        has[r] = true;
-        nb[r][0] = a.e[q]; nb[r][1] = a.h[q]; nb[r][2] = a.hu[q]; nb[r][3] = a.hv[q];
+        qn[r] = nc * NP2 + node;
+        nb[r][1] = a.h[qn[r]];
+    }
+    grid_dependency_wait();
+    if (valid) {
+        e = a.e[t]; hu0 = a.hu[t]; hv0 = a.hv[t];
+        if (a.Fx) { fx = a.Fx[t]; fy = a.Fy[t]; }
+    }
+#pragma unroll
+    for (int r = 0; r < Tl::NI; ++r) {
+        if (qn[r] < 0) continue;
+        nb[r][0] = a.e[qn[r]]; nb[r][2] = a.hu[qn[r]]; nb[r][3] = a.hv[qn[r]];
     }
     baro_tile_core<NP, FK, false>(
         T, G, valid, e, hu0, hv0, hb, fc, a.tdev, toff, false,
         [&](int r, double *q) {
-            if (!has[r]) return false;
+            if (qn[r] < 0) return false;
             q[0] = nb[r][0] + nb[r][1]; q[1] = nb[r][2]; q[2] = nb[r][3];
             return true;
         },
@@ -1487,6 +1506,7 @@ __device__ __forceinline__ void baro_pred_body(const BaroArgs &a, int64_t tile, 
 template <int NP, int FK, int CPB>
 __global__ void BARO_BOUNDS baro_pred_kernel(BaroArgs a, double dtb, double *k1e, double *k1u, double *k1v,
                                  double *es, double *us, double *vs) {
+    grid_launch_dependents();
     baro_pred_body<NP, FK, CPB>(a, blockIdx.x, a.toff, dtb, k1e, k1u, k1v, es, us, vs);
 }
 
@@ -1509,6 +1529,7 @@ template <int NP, int FK, int CPB>
 __global__ void BARO_BOUNDS baro_corr_kernel(BaroArgs a, double dtb, const double *k1e, const double *k1u,
                                  const double *k1v, double *e, double *hu, double *hv,
                                  double *esum, int first) {
+    grid_launch_dependents();
     baro_corr_body<NP, FK, CPB>(a, blockIdx.x, a.toff, dtb, k1e, k1u, k1v, e, hu, hv, esum, first);
 }
 
@@ -1633,6 +1654,7 @@ __global__ void baro_force_ens_kernel(BaroArgs a, BaroEns E, const double *dHU3,
 template <int NP, int FK, int CPB = BARO_CPB>
 __global__ void BARO_BOUNDS baro_pred_ens_kernel(BaroArgs a, BaroEns E, double *k1e, double *k1u,
                                                  double *k1v, double *es, double *us, double *vs) {
+    grid_launch_dependents();
     const int2 w = E.tiles[blockIdx.x];
     const EnsMember &m = E.mem[w.x];
     shift_baro(a, m, w.x);
@@ -1645,6 +1667,7 @@ template <int NP, int FK, int CPB = BARO_CPB>
 __global__ void BARO_BOUNDS baro_corr_ens_kernel(BaroArgs a, BaroEns E, const double *k1e, const double *k1u,
                                                  const double *k1v, double *e, double *hu, double *hv,
                                                  double *esum) {
+    grid_launch_dependents();
     const int2 w = E.tiles[blockIdx.x];
     const EnsMember &m = E.mem[w.x];
     shift_baro(a, m, w.x);
@@ -2521,6 +2544,11 @@ struct drf_dg {
         const char *tu = std::getenv("DRIFTER_B200_TUNE"), *pe = std::getenv("DRIFTER_B200_BARO_PERSISTENT");
         // sequence numbers hold 2^20 passes a launch
         if (view || (tu && tu[0] == '0') || (pe && pe[0]) || nsub >= (1 << 19)) return 0;
+        // With the pressure gradient on, a mixed-precision run amplifies a change of 1e-16 in the 2D
+        // state to the size of its FP32 noise within a few steps. There the form must not show: it
+        // has the per-pass kernels' bits with the Lax-Friedrichs flux from N = 2 on (elsewhere the
+        // compiler fuses some multiply-add differently, or the flux is hllc_flux_diff).
+        if (mixed && G.eos && !(G.flux2d == DRF_FLUX_LF && np >= 3)) return 0;
         int form = 0;
         dispatch_np(np, [&](auto npc) {
             constexpr int NP = decltype(npc)::value;
@@ -2594,13 +2622,12 @@ struct drf_dg {
                 DRF_LAUNCHED();
                 const double dtb = dt / nsub;
                 for (int m = 0; m < nsub; ++m) {
-                    baro_pred_kernel<NP, FK, CPB><<<nbt, bt, 0, stream>>>(
-                        baro<NP>(eta, HU, HV, true, m * dtb), dtb, k1[0], k1[1], k1[2], us[0], us[1], us[2]);
-                    DRF_LAUNCHED();
-                    baro_corr_kernel<NP, FK, CPB><<<nbt, bt, 0, stream>>>(
-                        baro<NP>(us[0], us[1], us[2], true, m * dtb + dtb), dtb, k1[0], k1[1], k1[2], eta,
-                        HU, HV, esum, m == 0);
-                    DRF_LAUNCHED();
+                    launch_overlapped(baro_pred_kernel<NP, FK, CPB>, nbt, bt, stream,
+                                      baro<NP>(eta, HU, HV, true, m * dtb), dtb, k1[0], k1[1], k1[2], us[0],
+                                      us[1], us[2]);
+                    launch_overlapped(baro_corr_kernel<NP, FK, CPB>, nbt, bt, stream,
+                                      baro<NP>(us[0], us[1], us[2], true, m * dtb + dtb), dtb, k1[0], k1[1],
+                                      k1[2], eta, HU, HV, esum, m == 0);
                 }
             });
         });
@@ -3513,6 +3540,11 @@ struct drf_ens {
         size_t smem;
     };
     std::vector<Group> groups;
+    // streams and events that the step graphs are captured with (a branch per further layer count);
+    // nothing is launched on them outside a capture
+    std::vector<cudaStream_t> branch;
+    cudaEvent_t ev_fork = nullptr;
+    std::vector<cudaEvent_t> ev_join;
     int nitems = 0, ntiles = 0, grid = 0;
     int64_t n3tot = 0, n2tot = 0;
     cudaStream_t stream = nullptr, own = nullptr;
@@ -3528,6 +3560,9 @@ struct drf_ens {
     }
     ~drf_ens() {
         drop_graphs();
+        for (auto &b : branch) cudaStreamDestroy(b);
+        for (auto &ev : ev_join) cudaEventDestroy(ev);
+        if (ev_fork) cudaEventDestroy(ev_fork);
         if (own) cudaStreamDestroy(own);
     }
 
@@ -3542,11 +3577,20 @@ struct drf_ens {
             StageArgs<T> a = m0->template stage_args<T>(src, dst, s, 0.0, 0, nullptr, nullptr, nullptr,
                                                         m0->eta, 0.0, s == 0);
             a.pf = 0;  // the work items are not in column order
-            for (const Group &g : groups) {
-                dg3d_stage_ens_kernel<T, NP><<<g.count, g.threads, g.smem, stream>>>(a, table.p, items.p + g.start,
-                                                                                     g.count);
+            // the layer counts' launches of a stage are independent: parallel branches of the step
+            // graph, so one's last wave shares the chip with the next
+            // (24 members, 5 heights: 1883 us a step one after the other, 1731 us)
+            if (groups.size() > 1) DRF_CUDA(cudaEventRecord(ev_fork, stream));
+            for (size_t k = 0; k < groups.size(); ++k) {
+                const Group &g = groups[k];
+                cudaStream_t st = k == 0 ? stream : branch[k - 1];
+                if (k > 0) DRF_CUDA(cudaStreamWaitEvent(st, ev_fork, 0));
+                dg3d_stage_ens_kernel<T, NP><<<g.count, g.threads, g.smem, st>>>(a, table.p, items.p + g.start,
+                                                                                 g.count);
                 DRF_LAUNCHED();
+                if (k > 0) DRF_CUDA(cudaEventRecord(ev_join[k - 1], st));
             }
+            for (size_t k = 1; k < groups.size(); ++k) DRF_CUDA(cudaStreamWaitEvent(stream, ev_join[k - 1], 0));
             src = dst;
         }
         if (baro_persist) {
@@ -3574,14 +3618,12 @@ struct drf_ens {
             DRF_LAUNCHED();
             for (int sub = 0; sub < nsub; ++sub) {
                 const BaroEns E{table.p, tiles.p, nsub, sub};
-                baro_pred_ens_kernel<NP, FK><<<ntiles, bt, 0, stream>>>(
-                    m0->template baro<NP>(m0->eta, m0->HU, m0->HV, true, 0.0), E, m0->k1[0], m0->k1[1],
-                    m0->k1[2], m0->us[0], m0->us[1], m0->us[2]);
-                DRF_LAUNCHED();
-                baro_corr_ens_kernel<NP, FK><<<ntiles, bt, 0, stream>>>(
-                    m0->template baro<NP>(m0->us[0], m0->us[1], m0->us[2], true, 0.0), E, m0->k1[0], m0->k1[1],
-                    m0->k1[2], m0->eta, m0->HU, m0->HV, m0->esum);
-                DRF_LAUNCHED();
+                launch_overlapped(baro_pred_ens_kernel<NP, FK>, ntiles, bt, stream,
+                                  m0->template baro<NP>(m0->eta, m0->HU, m0->HV, true, 0.0), E, m0->k1[0],
+                                  m0->k1[1], m0->k1[2], m0->us[0], m0->us[1], m0->us[2]);
+                launch_overlapped(baro_corr_ens_kernel<NP, FK>, ntiles, bt, stream,
+                                  m0->template baro<NP>(m0->us[0], m0->us[1], m0->us[2], true, 0.0), E, m0->k1[0],
+                                  m0->k1[1], m0->k1[2], m0->eta, m0->HU, m0->HV, m0->esum);
             }
         });
         const int64_t nfin = n2tot > (int64_t)mem.size() ? n2tot : (int64_t)mem.size();
@@ -3670,6 +3712,13 @@ int drf_ens_create(int nmembers, const drf_mesh_desc *meshes, const drf_dg_param
             if (e->groups.empty() || e->groups.back().nz != m.G.nz)
                 e->groups.push_back({i, 0, m.G.nz, m.stage_threads_generic(), m.smem});
             ++e->groups.back().count;
+        }
+        DRF_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
+        for (size_t k = 1; k < e->groups.size(); ++k) {
+            e->branch.push_back(nullptr);
+            DRF_CUDA(cudaStreamCreateWithFlags(&e->branch.back(), cudaStreamNonBlocking));
+            e->ev_join.push_back(nullptr);
+            DRF_CUDA(cudaEventCreateWithFlags(&e->ev_join.back(), cudaEventDisableTiming));
         }
         e->table.alloc(nmembers);
         DRF_CUDA(cudaMemcpy(e->table.p, e->htab.data(), nmembers * sizeof(EnsMember), cudaMemcpyHostToDevice));
