@@ -49,6 +49,24 @@ def test_vcycle_matches_oracle(n):
     assert rel(g.mg_apply(r), o.vcycle(r)) < 1e-11
 
 
+@pytest.mark.parametrize("n,coarsest,pre,post", [(18, 9, 1, 1), (20, 5, 1, 1), (22, 11, 1, 1), (40, 5, 1, 1),
+                                                 (18, 9, 2, 1), (20, 5, 0, 2)])
+def test_vcycle_color_steps_at_tile_edges(n, coarsest, pre, post):
+    """Grids whose last 8 x 4 tiles of the one-launch color step hold 2, 4, 6 and 8 columns; sweep
+    counts that start a level from zero, from a sweep before and from the coarse correction
+    alone (linear in r, and a contraction in the reference's form)."""
+    g, o = pair(n)
+    g.mg_setup(coarsest, pre, post)
+    r = np.random.default_rng(n).standard_normal(g.ndof)
+    z = g.mg_apply(r)
+    if (pre, post) == (1, 1):
+        o.mg_setup(coarsest)
+        assert rel(z, o.vcycle(r)) < 1e-11
+    assert rel(g.mg_apply(-2.0 * r), -2.0 * z) < 1e-11
+    x, k, relres = g.mg_apply_reference(r, tol=1e-6, max_vcycles=100)
+    assert relres < 1e-6 and k < 100
+
+
 @pytest.mark.parametrize("n", [4, 16, 32])
 def test_reference_mg_apply_matches_oracle(n):
     """BezierMultigridPreconditioner::apply as written (row-normalised restriction, one colour
