@@ -55,8 +55,9 @@ struct AmrArgs {
     // the LSRK stage form (amr_rhs_kernel<NP, true>): the mortar lifts added in the lift
     // kernel's order, then the mass inverse and res = A res + dt (-M^-1 R), Uout = U + B res
     const double *contrib;  // staged mortar lifts (null: no interfaces)
-    const int *lptr;        // lift entries of element e: lent[lptr[e] .. lptr[e + 1])
-    const int2 *lent;       // (row of contrib, face)
+    const unsigned *lptr;   // lift entries of element e: lent[lptr[e] .. lptr[e + 1])
+    const int2 *lent;       // (interface, 8 slot + face)
+    int slots;
     double *res, *Uout;
     double A, B, dt;
     int first;
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(amr_epb<NP>() * NP * NP, amr_min_ctas<NP>()) a
         if (a0 == 0 || a0 == N) ny = t[a0 == 0 ? 2 : 3];
         if (a1 == 0 || a1 == N) nz = t[a1 == 0 ? 4 : 5];
     }
-    int lift0 = 0, lift1 = 0;
+    unsigned lift0 = 0, lift1 = 0;
     if (STAGE && valid && a.lptr) {
         lift0 = a.lptr[e];
         lift1 = a.lptr[e + 1];
@@ -255,10 +256,10 @@ __global__ void __launch_bounds__(amr_epb<NP>() * NP * NP, amr_min_ctas<NP>()) a
     const size_t t = (size_t)e * NP3 + xo;
     if constexpr (STAGE) {
         // mortar lifts of the interfaces touching this element, in the lift kernel's order
-        for (int q = lift0; q < lift1; ++q) {
+        for (unsigned q = lift0; q < lift1; ++q) {
             const int2 en = a.lent[q];
-            const double *c = a.contrib + (size_t)en.x * NP2;
-            const int f = en.y, b = (f & 1) ? N : 0;
+            const double *c = a.contrib + ((size_t)en.x * a.slots + (en.y >> 3)) * NP2;
+            const int f = en.y & 7, b = (f & 1) ? N : 0;
             if (f < 2) {
                 const double v = c[l];
                 if (b == 0) r[0] += v;
@@ -506,7 +507,7 @@ struct drf_amr {
     DevBuf<double> U, R, res, out;
     int cur = 0;
     drf_mortar *mortar = nullptr;
-    DevBuf<int> lptr;   // the stage kernel's mortar lifts per element (AmrArgs::lptr, lent)
+    DevBuf<unsigned> lptr;  // the stage kernel's mortar lifts per element (AmrArgs::lptr, lent)
     DevBuf<int2> lent;
     // step graphs for each starting buffer (a step's five stages flip it)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -560,6 +561,7 @@ struct drf_amr {
             A.contrib = mortar ? L.contrib : nullptr;
             A.lptr = mortar ? lptr.p : nullptr;
             A.lent = lent.p;
+            A.slots = L.slots;
             A.A = AMR_LSRK_A[s]; A.B = AMR_LSRK_B[s]; A.dt = dt; A.first = s == 0;
             amr_dispatch(np, [&](auto npc) {
                 constexpr int NP = decltype(npc)::value;
@@ -710,13 +712,14 @@ int drf_amr_create(int order, int64_t n_elem, int64_t n_conf, const int64_t *con
             std::vector<int64_t> touched(L.n_touched), ptr(L.n_touched + 1);
             DRF_CUDA(cudaMemcpy(touched.data(), L.touched, L.n_touched * 8, cudaMemcpyDeviceToHost));
             DRF_CUDA(cudaMemcpy(ptr.data(), L.ptr, ptr.size() * 8, cudaMemcpyDeviceToHost));
-            std::vector<int> ent(3 * (size_t)ptr.back()), lp((size_t)n_elem + 1, 0);
+            DRF_CHECK(ptr.back() < ((int64_t)1 << 32), DRF_E_UNSUPPORTED, "AMR: too many interfaces");
+            std::vector<int> ent(3 * (size_t)ptr.back());
+            std::vector<unsigned> lp((size_t)n_elem + 1, 0);
             DRF_CUDA(cudaMemcpy(ent.data(), L.ent, ent.size() * 4, cudaMemcpyDeviceToHost));
-            DRF_CHECK(n_if * L.slots < ((int64_t)1 << 31), DRF_E_UNSUPPORTED, "AMR: too many interfaces");
             std::vector<int2> le((size_t)ptr.back());
             for (size_t q = 0; q < le.size(); ++q)
-                le[q] = make_int2(ent[3 * q] * L.slots + ent[3 * q + 1], ent[3 * q + 2]);
-            for (int64_t u = 0; u < L.n_touched; ++u) lp[touched[u] + 1] = (int)(ptr[u + 1] - ptr[u]);
+                le[q] = make_int2(ent[3 * q], 8 * ent[3 * q + 1] + ent[3 * q + 2]);
+            for (int64_t u = 0; u < L.n_touched; ++u) lp[touched[u] + 1] = (unsigned)(ptr[u + 1] - ptr[u]);
             for (int64_t e = 0; e < n_elem; ++e) lp[e + 1] += lp[e];
             h->lptr.alloc(lp.size());
             h->lent.alloc(le.size());
@@ -761,6 +764,7 @@ int drf_amr_download(drf_amr *h, double *U) {
         amr_check(h);
         DRF_CHECK(U, DRF_E_INVALID, "null argument");
         const size_t n = (size_t)h->n_elem * h->nd;
+        map_pages(U, n * 8);  // while the steps that were queued run
         DRF_CUDA(cudaMemcpyAsync(U, h->state(), n * 8, cudaMemcpyDeviceToHost, h->stream));
         DRF_CUDA(cudaStreamSynchronize(h->stream));
         DRF_CHECK(all_finite(U, n), DRF_E_NONFINITE, "non-finite state (the run blew up)");
@@ -783,6 +787,7 @@ int drf_amr_compute_rhs(drf_amr *h, int mode, int flux_kind, const double *a, co
             amr_massinv_kernel<NP><<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(n, h->R.p, h->out.p);
             DRF_LAUNCHED();
         });
+        map_pages(rhs, (size_t)n * 8);
         DRF_CUDA(cudaMemcpyAsync(rhs, h->out.p, n * 8, cudaMemcpyDeviceToHost, h->stream));
         DRF_CUDA(cudaStreamSynchronize(h->stream));
     });

@@ -2733,6 +2733,7 @@ void to_device(drf_dg *m, void *dst, const double *src) {
 }
 
 void from_device(drf_dg *m, double *dst, const void *src) {
+    map_pages(dst, (size_t)m->n3 * 8);
     if (!m->mixed) {
         DRF_CUDA(cudaMemcpyAsync(dst, src, m->n3 * 8, cudaMemcpyDeviceToHost, m->stream));
         DRF_CUDA(cudaStreamSynchronize(m->stream));

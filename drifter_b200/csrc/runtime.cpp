@@ -1,6 +1,13 @@
 // Host runtime of libdrifter_b200: error buffer, launch counter, LGL basis construction.
+#include <sys/mman.h>
+
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <system_error>
+#include <thread>
+#include <vector>
 
 #include "common.cuh"
 
@@ -24,10 +31,51 @@ int &capture_depth() {
     return d;
 }
 
+namespace {
+// fn(lo, hi) over [0, n) in equal parts on up to 8 host threads; on the calling thread alone where no
+// thread can be started
+template <class F>
+void on_host_threads(size_t n, F &&fn) {
+    const size_t nt = std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
+    const size_t part = (n + nt - 1) / nt;
+    std::vector<std::thread> th;
+    size_t lo = part;  // the first part is the calling thread's
+    try {
+        for (; lo < n; lo += part) th.emplace_back(fn, lo, std::min(n, lo + part));
+    } catch (const std::system_error &) {
+        fn(lo, n);
+    }
+    fn(size_t(0), std::min(n, part));
+    for (auto &t : th) t.join();
+}
+}  // namespace
+
 bool all_finite(const double *x, size_t n) {
-    for (size_t i = 0; i < n; ++i)
-        if (!std::isfinite(x[i])) return false;
-    return true;
+    auto part = [x](size_t lo, size_t hi) {
+        for (size_t i = lo; i < hi; ++i)
+            if (!std::isfinite(x[i])) return false;
+        return true;
+    };
+    // on host threads where one thread takes 5 ms and more (starting eight takes 0.1 ms to 1 ms)
+    if (n < ((size_t)1 << 23)) return part(0, n);
+    std::atomic<bool> ok{true};
+    on_host_threads(n, [&](size_t lo, size_t hi) {
+        if (!part(lo, hi)) ok = false;
+    });
+    return ok;
+}
+
+void map_pages(void *p, size_t bytes) {
+    constexpr size_t PAGE = 4096, MIN = (size_t)32 << 20;
+    if (bytes < MIN) return;
+    const uintptr_t lo = ((uintptr_t)p + PAGE - 1) / PAGE * PAGE, hi = ((uintptr_t)p + bytes) / PAGE * PAGE;
+    on_host_threads((hi - lo) / PAGE, [lo](size_t a, size_t b) {
+#ifdef MADV_POPULATE_WRITE
+        (void)madvise((void *)(lo + a * PAGE), (b - a) * PAGE, MADV_POPULATE_WRITE);
+#else
+        (void)madvise((void *)(lo + a * PAGE), (b - a) * PAGE, 23);  // Linux 5.14's number for it
+#endif
+    });
 }
 
 static void legendre(int n, double x, double &L, double &dL) {

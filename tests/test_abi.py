@@ -67,3 +67,14 @@ def test_nonfinite_input_rejected_without_gpu():
     p = np.array([9.81, 1025, 2e-4, 7.6e-4, 1, 1e-4, 1e-5, 1e-5])
     rc = L.drf_compat_modesplit_step(2, 1, 1.0, 2, dptr_array(arrs), dptr(h), dptr(f), dptr(p))
     assert rc == 4
+
+
+def test_nonfinite_value_at_the_end_of_a_large_array_rejected_without_gpu():
+    """Arrays of 2^23 values and more are looked through on several host threads."""
+    L = lib()
+    nel, nd = (1 << 20) + 3, 8
+    a = np.ones((nel, nd))
+    a[-1, -1] = np.inf
+    p = np.array([9.81, 1025, 2e-4, 7.6e-4, 1, 1e-4, 1e-5, 1e-5])
+    rc = L.drf_compat_modesplit_step(1, nel, 1.0, 2, dptr_array([a] * 12), dptr(a), dptr(a), dptr(p))
+    assert rc == 4
