@@ -1844,7 +1844,9 @@ __global__ void BARO_BOUNDS baro_subcycles_kernel(const __grid_constant__ BaroAr
 // between two buffers: a tile writes a buffer again two passes later, after it has read its
 // neighbours' traces of the pass between, which they publish after reading this buffer.
 // Sequence numbers grow from launch to launch (the epoch word), so no trace is taken for
-// another step's. The launch is cooperative (all CTAs resident) and every poll is bounded.
+// another step's: the epoch and the two other words are this form's own and live with the traces
+// (the grid-barrier form leaves other values in its words). The launch is cooperative (all CTAs
+// resident) and every poll is bounded.
 //
 // Bound by latency: an exchange and the dependent chain of a face flux (a reciprocal, a square
 // root) per pass, 1.5 us at C1 (256 columns, N = 3) against 3.3 us for a launch per pass.
@@ -1854,7 +1856,7 @@ struct ResidentArgs {
     const double *h, *f, *Fx, *Fy, *dHU3, *dHV3, *etbf;
     double *eta, *HU, *HV, *eta_avg, *corrU, *corrV, *corrR, *tdev;
     ulonglong2 *trace;  // [2][column][side][face node][e, hu, hv]: value, sequence number
-    unsigned *sync;     // [0] epoch, [1] CTAs finished, [2] abort; the last CTA leaves [1], [2] zero
+    unsigned *words;    // [0] epoch, [1] CTAs finished, [2] abort; the last CTA leaves [1], [2] zero
     int *err;
     int hold;  // failure-detection check: this CTA publishes no trace (-1: none)
     Geo G;
@@ -1909,7 +1911,7 @@ __global__ void __launch_bounds__(resident_cpb<NP>() * NP * NP, resident_ctas<NP
     const int tile = blockIdx.x, c = tile * CPB + lc;
     const bool valid = c < a.ncol;
     if (threadIdx.x < NP2) T.D[threadIdx.x] = cBs[NP].D[threadIdx.x];
-    const uint64_t seq0 = ((uint64_t) * (volatile unsigned *)&a.sync[0] + 1) << 20;
+    const uint64_t seq0 = ((uint64_t) * (volatile unsigned *)&a.words[0] + 1) << 20;
     const size_t t = (size_t)c * NP2 + an;
     const int ex = c % G.nx, ey = c / G.nx;
     double hb = 0.0, fc = 0.0, xe = 0.0, xu = 0.0, xv = 0.0;  // x: the state Phi is evaluated at
@@ -1970,7 +1972,7 @@ __global__ void __launch_bounds__(resident_cpb<NP>() * NP * NP, resident_ctas<NP
                     nb[r][1] = trace_get(w + 1, q1);
                     nb[r][2] = trace_get(w + 2, q2);
                     if (q0 == want && q1 == want && q2 == want) break;
-                    if (it > (1 << 20) || ((it & 255) == 255 && *(volatile unsigned *)&a.sync[2] != 0u)) {
+                    if (it > (1 << 20) || ((it & 255) == 255 && *(volatile unsigned *)&a.words[2] != 0u)) {
                         fail = true;
                         break;
                     }
@@ -2028,18 +2030,18 @@ __global__ void __launch_bounds__(resident_cpb<NP>() * NP * NP, resident_ctas<NP
         a.corrR[t] = tracer_volume_correction(xe, a.etbf[t], hb);
     }
     if (!ok && threadIdx.x == 0) {
-        atomicExch(&a.sync[2], 1u);
+        atomicExch(&a.words[2], 1u);
         atomicExch(a.err, DRF_E_TIMEOUT);
     }
     // the last CTA to finish: the clock advances once every CTA is past its last read of it
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(&a.sync[1], 1u) == gridDim.x - 1) {
+        if (atomicAdd(&a.words[1], 1u) == gridDim.x - 1) {
             __threadfence();
-            a.sync[0] += 1;
-            a.sync[1] = 0;
-            if (atomicExch(&a.sync[2], 0u) == 0u) a.tdev[0] = a.tdev[0] + a.dt;
+            a.words[0] += 1;
+            a.words[1] = 0;
+            if (atomicExch(&a.words[2], 0u) == 0u) a.tdev[0] = a.tdev[0] + a.dt;
         }
     }
 }
@@ -2352,9 +2354,10 @@ struct drf_dg {
     // graphs are built, from DRIFTER_B200_DEBUG_HOLD_ARRIVAL
     int debug_hold = -1;
     // resident form of the barotropic step (resident_form; fixed when the step graphs are
-    // built) and its trace slots
+    // built), its trace slots and after them its words (ResidentArgs), zeroed once, together
     int baro_res = 0;
     DevBuf<ulonglong2> trace;
+    size_t trace_slots() const { return (size_t)2 * ncol * 4 * np * 3; }
     // 3D arrays: q3p + (array * n3s + node) * tsz; n3s = n3 for a model that owns its memory,
     // the pool length for an ensemble member (a view into the ensemble's pools)
     unsigned char *q3p = nullptr;
@@ -2558,7 +2561,7 @@ struct drf_dg {
             });
         });
         if (form && !trace.n) {
-            trace.alloc((size_t)2 * ncol * 4 * np * 3);
+            trace.alloc(trace_slots() + 1);
             DRF_CUDA(cudaMemsetAsync(trace.p, 0, trace.n * sizeof(ulonglong2), stream));
         }
         return form;
@@ -2590,7 +2593,7 @@ struct drf_dg {
             r.h = h; r.f = f; r.Fx = Fx; r.Fy = Fy; r.dHU3 = dHU3; r.dHV3 = dHV3; r.etbf = etb[0];
             r.eta = eta; r.HU = HU; r.HV = HV; r.eta_avg = eta_avg;
             r.corrU = corrU; r.corrV = corrV; r.corrR = corrR; r.tdev = tdev;
-            r.trace = trace.p; r.sync = syncbuf.p; r.err = err; r.hold = debug_hold; r.G = G;
+            r.trace = trace.p; r.words = (unsigned *)(trace.p + trace_slots()); r.err = err; r.hold = debug_hold; r.G = G;
             dispatch_flux(G.flux2d, [&](auto fk) {
                 constexpr int FK = decltype(fk)::value;
                 if (baro_res == 1) launch_resident<NP, FK, false>(r, stream);

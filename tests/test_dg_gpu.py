@@ -356,6 +356,42 @@ def test_resident_barotropic_step_equals_per_pass_launches(monkeypatch, order, n
         assert relerr(a[k], b[k]) <= 1e-11, (k, relerr(a[k], b[k]))
 
 
+# 9 x 7 columns: at N = 1 the grid-barrier launch has as many CTAs as the resident one (8) or more, at
+# N = 3 as many (32) or fewer; 1 and 2 subcycles rewrite no trace slot within a step
+@pytest.mark.parametrize("order,nsub", [(1, 1), (1, 2), (3, 1), (3, 2), (3, 6)])
+def test_one_model_through_all_barotropic_forms(monkeypatch, order, nsub):
+    """The form is chosen anew whenever the step graphs are rebuilt, here by a change of dt. A model
+    that goes through all of them keeps its clock exactly and its state to the 1e-10 of the oracle
+    comparisons against one that stays with a launch per pass (the forms agree to 1e-11 over two
+    steps)."""
+    case = _tidal_small("fp64", order=order, nx=9, ny=7, nz=1)
+    dt0 = case["dt"] * nsub / case["nsub"] * min(1.0, 5.0 / 9.0)
+    models = []
+    for _ in range(2):
+        m = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+        m.upload_state(case["q"], case["eta"])
+        models.append(m)
+    launches = {None: 7, "1": 6, "0": 5 + 2 + 2 * nsub}
+    for k, form in enumerate((None, "1", None, "0", "1", "1", None, None)):
+        dt = dt0 * (1.0 - 0.02 * k)
+        for m, env in zip(models, (form, "0")):
+            if env is None:
+                monkeypatch.delenv("DRIFTER_B200_BARO_PERSISTENT", raising=False)
+            else:
+                monkeypatch.setenv("DRIFTER_B200_BARO_PERSISTENT", env)
+            m.step(dt, nsub, 0)  # builds the step graphs
+            before = launch_count()
+            m.step(dt, nsub, 3)
+            m.sync()
+            assert launch_count() - before == 3 * launches[env], (k, env)
+        a, b = (m.download_state() for m in models)
+        assert a["t"] == b["t"], k
+        for v in ("eta", "HU", "HV", "eta_avg", "Hu", "HT"):
+            assert relerr(a[v], b[v]) <= 1e-10, (k, form, v, relerr(a[v], b[v]))
+    for m in models:
+        m.close()
+
+
 def test_resident_barotropic_steps_of_two_models_at_once():
     """Two models step on their own streams from two host threads, their resident launches in
     flight together: each ends where it does alone."""
