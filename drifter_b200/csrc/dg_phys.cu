@@ -2371,6 +2371,11 @@ struct drf_dg {
            *corrV = nullptr, *etb[2] = {}, *rese = nullptr, *corrR = nullptr;
     int cur = 0;
     bool pending = false;  // a transport correction in corrU/corrV is not yet in q(cur)
+    // A device-side wait gave up: CTAs that finished have written their part of the new state, the
+    // others have not. Nothing steps or reads such a state until the next upload. (Single models;
+    // unreported: the status of a step before an upload, still owed to the caller.)
+    bool torn = false;
+    int unreported = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     uint64_t graph_kernels[2] = {0, 0};  // kernel nodes of each step graph
     double graph_dt = 0.0;
@@ -2750,15 +2755,26 @@ void from_device(drf_dg *m, double *dst, const void *src) {
 
 void check_model(drf_dg *m) { DRF_CHECK(m != nullptr, DRF_E_INVALID, "null model handle"); }
 
-// surfaces a status word set on the device (a bounded wait that gave up)
-void check_device_status(drf_dg *m) {
+// a model whose state may be stepped or read
+void check_state(drf_dg *m) {
+    check_model(m);
+    DRF_CHECK(!m->torn, DRF_E_TIMEOUT, "the state was lost when a device-side wait gave up: upload one");
+}
+
+// takes the status word set on the device (a bounded wait that gave up), leaving it zero
+int take_device_status(drf_dg *m) {
     int st = 0;
     DRF_CUDA(cudaMemcpyAsync(&st, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     DRF_CUDA(cudaStreamSynchronize(m->stream));
-    if (st != 0) {
-        DRF_CUDA(cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
-        throw Error(st, "a device-side wait gave up (status " + std::to_string(st) + ")");
-    }
+    if (st != 0) DRF_CUDA(cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
+    return st;
+}
+
+void check_device_status(drf_dg *m) {
+    int st = take_device_status(m);
+    if (st != 0 && !m->view) m->torn = true;
+    if (st == 0) std::swap(st, m->unreported);
+    if (st != 0) throw Error(st, "a device-side wait gave up (status " + std::to_string(st) + ")");
 }
 
 }  // namespace
@@ -3049,13 +3065,17 @@ int drf_dg_upload_state(drf_dg *m, const double *const *q4, const double *eta, d
         m->pending = false;
         DRF_CUDA(cudaStreamSynchronize(m->stream));
         m->drop_graphs();
+        if (!m->view) {  // a status that is still set is that of the state replaced here
+            if (const int st = take_device_status(m)) m->unreported = st;
+            m->torn = false;
+        }
     });
 }
 
 int drf_dg_download_state(drf_dg *m, double *const *q4, double *eta, double *HU, double *HV,
                           double *eta_avg, double *t) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         m->materialize();
         check_device_status(m);
         if (q4)
@@ -3076,7 +3096,7 @@ int drf_dg_download_state(drf_dg *m, double *const *q4, double *eta, double *HU,
 // snapshot waits for the previous copy.
 int drf_dg_output_stage(drf_dg *m, double *const *q4, double *eta, double *HU, double *HV) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         DRF_CHECK(!m->view, DRF_E_INVALID, "stage ensemble members' output through their ensemble's stream");
         if (!m->ostream) {
             DRF_CUDA(cudaStreamCreateWithFlags(&m->ostream, cudaStreamNonBlocking));
@@ -3132,7 +3152,7 @@ int drf_dg_output_wait(drf_dg *m, double *t) {
 
 int drf_dg_compute_rhs(drf_dg *m, double *const *r4, double *omega, double *deta) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         m->materialize();
         void *rout[4] = {m->tmp(0), m->tmp(1), m->tmp(2), m->tmp(3)};
         m->with_types([&](auto tv, auto npc) {
@@ -3153,7 +3173,7 @@ int drf_dg_compute_rhs(drf_dg *m, double *const *r4, double *omega, double *deta
 int drf_dg_compute_rhs2d(drf_dg *m, const double *Fx, const double *Fy, double time, double *ke,
                          double *khu, double *khv) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         DRF_CHECK(Fx && Fy && ke && khu && khv, DRF_E_INVALID, "null argument");
         DRF_CUDA(cudaMemcpyAsync(m->Fx, Fx, m->n2 * 8, cudaMemcpyHostToDevice, m->stream));
         DRF_CUDA(cudaMemcpyAsync(m->Fy, Fy, m->n2 * 8, cudaMemcpyHostToDevice, m->stream));
@@ -3179,7 +3199,7 @@ int drf_dg_compute_rhs2d(drf_dg *m, const double *Fx, const double *Fy, double t
 
 int drf_dg_step_modesplit(drf_dg *m, double dt, int nsub, int nsteps) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         DRF_CHECK(!m->view, DRF_E_INVALID, "ensemble members are stepped together (drf_ens_step)");
         DRF_CHECK(nsub >= 1, DRF_E_INVALID, "nsub must be >= 1");
         DRF_CHECK(dt > 0.0 && std::isfinite(dt), DRF_E_INVALID, "dt must be positive");
@@ -3215,7 +3235,7 @@ int drf_dg_step_modesplit(drf_dg *m, double dt, int nsub, int nsteps) {
 
 int drf_dg_rk_step(drf_dg *m, int scheme, double dt, int nsteps) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         DRF_CHECK(scheme >= 0 && scheme <= 5, DRF_E_INVALID, "unknown RK scheme");
         DRF_CHECK(dt > 0.0 && std::isfinite(dt), DRF_E_INVALID, "dt must be positive");
         m->materialize();
@@ -3351,7 +3371,7 @@ int drf_dg_rk_step(drf_dg *m, int scheme, double dt, int nsteps) {
 
 int drf_dg_diagnostics(drf_dg *m, double *out10) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         DRF_CHECK(out10, DRF_E_INVALID, "null output");
         int dev = 0, nsm = 0;
         DRF_CUDA(cudaGetDevice(&dev));
@@ -3482,7 +3502,7 @@ int drf_dg_set_forcing(drf_dg *m, const double *taux, const double *tauy) {
 
 int drf_dg_download_surface(drf_dg *m, double *eta) {
     return guard([&] {
-        check_model(m);
+        check_state(m);
         DRF_CHECK(eta, DRF_E_INVALID, "null argument");
         DRF_CUDA(cudaMemcpyAsync(eta, m->eta, m->n2 * 8, cudaMemcpyDeviceToHost, m->stream));
         DRF_CUDA(cudaStreamSynchronize(m->stream));

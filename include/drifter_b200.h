@@ -120,6 +120,10 @@ int drf_dg_create(const drf_mesh_desc *mesh, const drf_dg_params *params, const 
 int drf_dg_destroy(drf_dg *m);
 /* Uses the given cudaStream_t for all work of this model (NULL = the model's own stream). */
 int drf_dg_set_stream(drf_dg *m, void *cuda_stream);
+/* Waits for the model's work and reports a status set on the device: DRF_E_TIMEOUT once when a
+ * bounded device wait gave up. The state is incomplete then, and every call that steps or reads it
+ * returns DRF_E_TIMEOUT until drf_dg_upload_state (single models; drf_dg_download_state,
+ * drf_dg_output_wait and drf_dg_time_copy report the status as well). */
 int drf_dg_sync(drf_dg *m);
 
 /* Host FP64 state in/out. q = {Hu, Hv, HT, HS} 3D fields, eta 2D. On upload the barotropic

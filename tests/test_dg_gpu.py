@@ -445,6 +445,56 @@ def test_bounded_trace_wait_gives_up_and_the_model_stays_usable(monkeypatch):
         assert relerr(a[k], b[k]) <= 1e-11, k
 
 
+@pytest.mark.parametrize("persistent", [None, "1"])
+def test_state_of_a_step_that_gave_up_is_refused_until_the_next_upload(monkeypatch, persistent):
+    """A step whose waits gave up leaves the tiles that finished at the new state and the others at
+    the old one. It is reported once; calls that step or read that state then return DRF_E_TIMEOUT,
+    and after an upload the same handle agrees with the per-pass form. A step that gave up just
+    before an upload is still reported, once, and does not count against the new state."""
+    from drifter_b200 import DrfError
+    case = _tidal_small("fp64", nx=9, ny=7)
+    if persistent:
+        monkeypatch.setenv("DRIFTER_B200_BARO_PERSISTENT", persistent)
+    m = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+
+    def times_out(call):
+        with pytest.raises(DrfError) as ei:
+            call()
+        assert ei.value.code == 6  # DRF_E_TIMEOUT
+
+    def step_that_gives_up():
+        monkeypatch.setenv("DRIFTER_B200_DEBUG_HOLD_ARRIVAL", "0")
+        m.upload_state(case["q"], case["eta"])  # drops the step graphs
+        m.step(case["dt"], case["nsub"], 1)
+        monkeypatch.delenv("DRIFTER_B200_DEBUG_HOLD_ARRIVAL")
+
+    step_that_gives_up()
+    times_out(m.sync)
+    m.sync()  # reported, and the status word cleared
+    z = np.zeros(case["cfg"].n2)
+    out = {"eta": np.zeros(case["cfg"].n2)}
+    for call in (lambda: m.step(case["dt"], case["nsub"], 1), lambda: m.rk_step("ssp3", 1.0, 1), m.download_state,
+                 m.download_surface, m.diagnostics, m.compute_rhs, lambda: m.compute_rhs2d(z, z, 0.0),
+                 lambda: m.output_stage(out)):
+        times_out(call)
+    step_that_gives_up()
+    m.upload_state(case["q"], case["eta"])
+    times_out(m.sync)
+    m.sync()
+    m.step(case["dt"], case["nsub"], 2)
+    a = m.download_state()
+    m.close()
+    monkeypatch.setenv("DRIFTER_B200_BARO_PERSISTENT", "0")
+    per = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+    per.upload_state(case["q"], case["eta"])
+    per.step(case["dt"], case["nsub"], 2)
+    b = per.download_state()
+    per.close()
+    assert a["t"] == b["t"]
+    for k in ("eta", "HU", "HV", "Hu", "HT"):
+        assert relerr(a[k], b[k]) <= 1e-11, k
+
+
 def test_bounded_grid_barrier_wait_gives_up_and_the_model_stays_usable(monkeypatch):
     """Failure detection without a GPU fault. With DRIFTER_B200_DEBUG_HOLD_ARRIVAL=0 the
     persistent barotropic launch's CTA 0 withholds its arrival at the first grid barrier, so no
