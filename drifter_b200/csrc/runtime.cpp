@@ -5,7 +5,6 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -32,8 +31,8 @@ int &capture_depth() {
 }
 
 namespace {
-// fn(lo, hi) over [0, n) in equal parts on up to 8 host threads; on the calling thread alone where no
-// thread can be started
+// fn(lo, hi) over [0, n) in equal parts on up to 8 host threads; what no thread can be started for (no
+// thread or no memory for one to be had) is done by the calling one
 template <class F>
 void on_host_threads(size_t n, F &&fn) {
     const size_t nt = std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
@@ -41,8 +40,9 @@ void on_host_threads(size_t n, F &&fn) {
     std::vector<std::thread> th;
     size_t lo = part;  // the first part is the calling thread's
     try {
+        th.reserve(nt);
         for (; lo < n; lo += part) th.emplace_back(fn, lo, std::min(n, lo + part));
-    } catch (const std::system_error &) {
+    } catch (const std::exception &) {
         fn(lo, n);
     }
     fn(size_t(0), std::min(n, part));

@@ -2,6 +2,8 @@
 and rejects bad arguments with status codes before touching the GPU."""
 import ctypes as C
 import os
+import shutil
+import subprocess
 
 import numpy as np
 import pytest
@@ -78,3 +80,17 @@ def test_nonfinite_value_at_the_end_of_a_large_array_rejected_without_gpu():
     p = np.array([9.81, 1025, 2e-4, 7.6e-4, 1, 1e-4, 1e-5, 1e-5])
     rc = L.drf_compat_modesplit_step(1, nel, 1.0, 2, dptr_array([a] * 12), dptr(a), dptr(a), dptr(p))
     assert rc == 4
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no host C++ compiler")
+def test_failing_allocation_while_host_threads_start_ends_in_a_status(tmp_path):
+    """Where no memory is had for another host thread, the calling one does the rest: the same
+    status, and the process lives."""
+    root = os.path.dirname(_abi.HERE)
+    exe = str(tmp_path / "alloc_failure_check")
+    subprocess.run(["g++", "-std=c++20", "-O2", "-Wall", "-Wextra", "-Werror", "-I", os.path.join(root, "include"),
+                    os.path.join(root, "tests", "cpp", "alloc_failure_check.cpp"), "-L", _abi.HERE,
+                    "-ldrifter_b200", f"-Wl,-rpath,{_abi.HERE}", "-o", exe], check=True, capture_output=True, text=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    assert set(r.stdout.split()) == {"4"}, r.stdout
