@@ -1184,6 +1184,7 @@ struct drf_bz {
     DevBuf<int> ctl;
     struct Lv {
         DevBuf<double> K, rho, binv, x, b, r;
+        ElemOp op;                // K again, by value, for the tile kernel's parameter
         DevBuf<int> fc0, cf0;     // transfer tables from the next coarser level (TransferDev)
         DevBuf<double> fw, cw, rs;
         int n = 0, nd = 0;
@@ -1240,10 +1241,7 @@ struct drf_bz {
         constexpr int TI = 32, TJ = 8;
         const LevelDev L = levdev(l);
         const dim3 grid((unsigned)((L.n + TI - 1) / TI), (unsigned)((L.n + TJ - 1) / TJ));
-        ElemOp op;
-        for (int a = 0; a < 16; ++a)
-            for (int k = 0; k < 16; ++k) op.K[16 * k + a] = H.levels[l].K[16 * a + k];
-        bz_apply_tile_kernel<TI, TJ><<<grid, TI * TJ, 0, stream>>>(op, L, xin, bin, yout, mode, pt, stop);
+        bz_apply_tile_kernel<TI, TJ><<<grid, TI * TJ, 0, stream>>>(lv[l].op, L, xin, bin, yout, mode, pt, stop);
         DRF_LAUNCHED();
         return (int)(grid.x * grid.y);
     }
@@ -1883,7 +1881,9 @@ int drf_bz_create(const drf_bz_grid_desc *g, const double *dgauss, drf_bz **out)
         auto &F = h->lv[0];
         F.n = g->nx;
         F.nd = 3 * g->nx + 1;
-        up(F.K, transposed16(h->H.levels.back().K, 1));
+        const std::vector<double> kt = transposed16(h->H.levels.back().K, 1);
+        up(F.K, kt);
+        std::copy(kt.begin(), kt.end(), F.op.K);
         up(F.rho, h->H.levels.back().rho);
         F.binv.alloc(9 * 256);
         DRF_CUDA(cudaMemset(F.binv.p, 0, 9 * 256 * 8));
@@ -2042,6 +2042,7 @@ int drf_mg_setup(drf_bz *h, int coarsest_n, int pre, int post) {
             lv[l].nd = Lh.nd;
             const std::vector<double> kt = transposed16(Lh.K, 1);
             up(lv[l].K, kt);
+            std::copy(kt.begin(), kt.end(), lv[l].op.K);
             up(lv[l].rho, Lh.rho);
             std::vector<double> bi =
                 Lh.binv.empty() ? std::vector<double>(9 * 256, 0.0) : transposed16(Lh.binv.data(), 9);

@@ -67,6 +67,37 @@ def test_vcycle_color_steps_at_tile_edges(n, coarsest, pre, post):
     assert relres < 1e-6 and k < 100
 
 
+@pytest.mark.parametrize("before", [None, 4])
+def test_multigrid_setup_that_finds_no_memory_leaves_the_operator(before):
+    """drf_mg_setup on a full device returns DRF_E_NOMEM; the smoother, with no hierarchy or one of
+    another depth before, applies and solves as it did."""
+    import torch
+    from drifter_b200 import DrfError
+    n = 256
+    g = BezierSmoother(n, n, 5000.0, 5000.0, fbm(n), lam=1.0, ridge_epsilon=1e-4)
+    kind = "jacobi" if before is None else "mg"
+    if before:
+        g.mg_setup(before)
+    v = np.random.default_rng(4).standard_normal(g.ndof)
+    y, (x, info) = g.apply_Q(v), g.solve(kind, tol=1e-8, maxit=20000)
+    torch.cuda.synchronize()
+    full, size = [], 1 << 37
+    while size >= 1 << 20:  # all but about 1 MB; the finest level's array takes 4.7 MB
+        try:
+            full.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            size //= 2
+    with pytest.raises(DrfError) as ei:
+        g.mg_setup(8)
+    assert ei.value.code == 3  # DRF_E_NOMEM
+    full.clear()
+    torch.cuda.empty_cache()
+    assert np.array_equal(g.apply_Q(v), y)
+    x2, info2 = g.solve(kind, tol=1e-8, maxit=20000)
+    assert info2["iters"] == info["iters"] and np.array_equal(x2, x)
+    g.close()
+
+
 @pytest.mark.parametrize("n", [4, 16, 32])
 def test_reference_mg_apply_matches_oracle(n):
     """BezierMultigridPreconditioner::apply as written (row-normalised restriction, one colour
