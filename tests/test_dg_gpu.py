@@ -281,6 +281,32 @@ def test_autotuned_barotropic_tile_matches_default_tile(monkeypatch):
         assert relerr(a[k], b[k]) <= 1e-15, k
 
 
+@pytest.mark.parametrize("order,nx,ny", [(1, 9, 7), (3, 9, 7), (4, 21, 19)])
+def test_tuned_tile_of_the_per_pass_launches_equals_the_default_tile(monkeypatch, order, nx, ny):
+    """The launches per pass at the tile that the autotuner picked, whichever it is, give the bits of
+    the default tile (8 columns): every tile does the same arithmetic per 2D node. (A model of this
+    size takes the resident form, which has no such tile, unless the launch form is fixed.)"""
+    case = _tidal_small("fp64", order=order, nx=nx, ny=ny)
+    case["dt"] *= min(1.0, 5.0 / max(nx, ny))
+    monkeypatch.setenv("DRIFTER_B200_BARO_PERSISTENT", "0")
+    out = []
+    for tune in (None, "0"):
+        if tune:
+            monkeypatch.setenv("DRIFTER_B200_TUNE", tune)
+        m = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+        m.upload_state(case["q"], case["eta"])
+        m.step(case["dt"], case["nsub"], 0)
+        before = launch_count()
+        m.step(case["dt"], case["nsub"], 2)
+        m.sync()
+        assert launch_count() - before == 2 * (5 + 2 + 2 * case["nsub"])
+        assert m.tuning()["baro_cols_per_cta"] in ((2, 4, 8, 16) if tune is None else (8,))
+        out.append(m.download_state())
+        m.close()
+    for k in ("eta", "HU", "HV", "eta_avg", "Hu", "HT"):
+        assert np.array_equal(out[0][k], out[1][k]), k
+
+
 @pytest.mark.parametrize("precision,flux2d,nsub", [("fp64", "lf", 20), ("fp64", "hllc", 1), ("fp64", "roe", 3),
                                                     ("mixed", "lf", 20)])
 def test_persistent_barotropic_step_agrees_with_per_pass_launches(monkeypatch, precision, flux2d, nsub):
