@@ -1207,46 +1207,6 @@ __device__ __forceinline__ void lf_minus_phys(const double UL[3], double ihL, do
     }
 }
 
-// d = F*(U-, U+, n) - F(U-).n of the HLLC flux for a face normal along an axis, in the face's own components:
-// U = (h, hn, ht) with hn, ht the momentum along and across the axis, sg = +-1 the outward
-// direction along it, iL = 1 / h- (clamped as below). The interior flux is taken out of F*
-// algebraically, which also takes out the cancellation of their 0.5 g h^2. Same states, speeds and
-// branches as sw_flux; one division per state and speed instead of seven and more. For the resident
-// form, whose passes wait for the longest chain (23 x 17 columns at N = 2: 184 us a step against
-// 208 us with F* and F- formed separately); a launch per pass gains 2%, and keeps sw_flux.
-__device__ __forceinline__ double wet(double h) { return h < 1e-10 ? 1e-10 : h; }
-__device__ __forceinline__ void hllc_flux_diff(const double L[3], double iL, const double R[3], double sg, double g,
-                                               double d[3]) {
-    const double hL = wet(L[0]), hR = wet(R[0]), iR = 1.0 / hR;
-    const double nL = sg * L[1], nR = sg * R[1];  // outward momenta
-    const double uL = nL * iL, uR = nR * iR;      // outward velocities
-    const double vL = L[2] * iL, vR = R[2] * iR;
-    const double dh = R[0] - L[0], dn = nR - nL, dt = R[2] - L[2];
-    const double cR = sqrt(g * hR), cL = sqrt(g * hL);
-    // F+ - F-: mass, outward momentum, tangential momentum
-    const double gh = 0.5 * g * (hR - hL) * (hR + hL);
-    const double dFn = nR * uR - nL * uL + gh;
-    const double dFt = nR * vR - nL * vL;
-    double dN;
-    const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
-    const double mL = hL * (SL - uL), mR = hR * (SR - uR), den = mL - mR;
-    const double Ss = fabs(den) > 1e-10 ? (uL * mL - uR * mR + gh) / den : 0.5 * (uL + uR);
-    if (SL >= 0) {
-        d[0] = dN = d[2] = 0.0;
-    } else if (SR <= 0) {
-        d[0] = dn; dN = dFn; d[2] = dFt;
-    } else {
-        const bool left = Ss >= 0;
-        const double S = left ? SL : SR, hs = (left ? mL : mR) / (S - Ss);
-        const double *K = left ? L : R;
-        d[0] = S * (hs - wet(K[0]));
-        dN = S * (hs * Ss - (left ? nL : nR));
-        d[2] = S * (hs * (left ? vL : vR) - K[2]);
-        if (!left) { d[0] += dn; dN += dFn; d[2] += dFt; }
-    }
-    d[1] = sg * dN;
-}
-
 // Register budget of the subcycle kernels: 800 resident threads per SM (80 registers) for up to
 // 5 x 5 nodes per column, 576 (112 registers) for 6 x 6, whatever the tile.
 constexpr int baro_min_blocks(int threads, int np) {
@@ -1325,13 +1285,7 @@ __device__ __forceinline__ bool baro_tile_core(BaroTile<NP, CPB> &T, const Geo &
         } else if (FK == DRF_FLUX_LF) {
             lf_minus_phys(UL, T.I[ln], sqrt(G.g * (HL < 1e-10 ? 1e-10 : HL)), UR, nx, ny, G.g, d);
         } else {
-            // in the face's components: along the axis, then across it
-            const bool ax = s <= 1;
-            const double L[3] = {HL, ax ? UL[1] : UL[2], ax ? UL[2] : UL[1]};
-            const double R[3] = {UR[0], ax ? UR[1] : UR[2], ax ? UR[2] : UR[1]};
-            double q[3];
-            hllc_flux_diff(L, HL < 1e-10 ? 1e10 : T.I[ln], R, (s & 1) ? 1.0 : -1.0, G.g, q);
-            d[0] = q[0]; d[1] = ax ? q[1] : q[2]; d[2] = ax ? q[2] : q[1];
+            hllc_flux_diff_side(UL, T.I[ln], UR, s, G.g, d);
         }
         double *o = T.F + (lc * NF + it) * 3;
         o[0] = d[0]; o[1] = d[1]; o[2] = d[2];

@@ -71,6 +71,57 @@ __device__ __forceinline__ void sw_flux_hllc(const double UL[3], const double UR
     }
 }
 
+// d = F*(U-, U+, n) - F(U-).n of the HLLC flux for a face normal along an axis, in the face's own
+// components: U = (h, hn, ht) with hn, ht the momentum along and across the axis, sg = +-1 the outward
+// direction along it, iL = 1 / h- (clamped as below). The interior flux is taken out of F*
+// algebraically, which also takes out the cancellation of their 0.5 g h^2. Same states, speeds and
+// branches as sw_flux_hllc; one division per state and speed instead of seven and more. For the resident
+// barotropic form, whose passes wait for the longest chain (23 x 17 columns at N = 2: 184 us a step
+// against 208 us with F* and F- formed separately); a launch per pass gains 2%, and keeps sw_flux.
+__device__ __forceinline__ double wet(double h) { return h < 1e-10 ? 1e-10 : h; }
+__device__ __forceinline__ void hllc_flux_diff(const double L[3], double iL, const double R[3], double sg, double g,
+                                               double d[3]) {
+    const double hL = wet(L[0]), hR = wet(R[0]), iR = 1.0 / hR;
+    const double nL = sg * L[1], nR = sg * R[1];  // outward momenta
+    const double uL = nL * iL, uR = nR * iR;      // outward velocities
+    const double vL = L[2] * iL, vR = R[2] * iR;
+    const double cR = sqrt(g * hR), cL = sqrt(g * hL);
+    // F+ - F-: mass, outward momentum, tangential momentum
+    const double gh = 0.5 * g * (hR - hL) * (hR + hL);
+    const double dn = nR - nL;
+    const double dFn = nR * uR - nL * uL + gh;
+    const double dFt = nR * vR - nL * vL;
+    double dN;
+    const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
+    const double mL = hL * (SL - uL), mR = hR * (SR - uR), den = mL - mR;
+    const double Ss = fabs(den) > 1e-10 ? (uL * mL - uR * mR + gh) / den : 0.5 * (uL + uR);
+    if (SL >= 0) {
+        d[0] = dN = d[2] = 0.0;
+    } else if (SR <= 0) {
+        d[0] = dn; dN = dFn; d[2] = dFt;
+    } else {
+        const bool left = Ss >= 0;
+        const double S = left ? SL : SR, hs = (left ? mL : mR) / (S - Ss);
+        const double *K = left ? L : R;
+        d[0] = S * (hs - wet(K[0]));
+        dN = S * (hs * Ss - (left ? nL : nR));
+        d[2] = S * (hs * (left ? vL : vR) - K[2]);
+        if (!left) { d[0] += dn; dN += dFn; d[2] += dFt; }
+    }
+    d[1] = sg * dN;
+}
+// the same across side s of an element (0 -x, 1 +x, 2 -y, 3 +y), states and d in (h, hu, hv);
+// ihL = 1 / h-, not clamped
+__device__ __forceinline__ void hllc_flux_diff_side(const double UL[3], double ihL, const double UR[3], int s, double g,
+                                                    double d[3]) {
+    const bool ax = s <= 1;
+    const double L[3] = {UL[0], ax ? UL[1] : UL[2], ax ? UL[2] : UL[1]};
+    const double R[3] = {UR[0], ax ? UR[1] : UR[2], ax ? UR[2] : UR[1]};
+    double q[3];
+    hllc_flux_diff(L, UL[0] < 1e-10 ? 1e10 : ihL, R, (s & 1) ? 1.0 : -1.0, g, q);
+    d[0] = q[0]; d[1] = ax ? q[1] : q[2]; d[2] = ax ? q[2] : q[1];
+}
+
 __device__ __forceinline__ void sw_flux_roe(const double UL[3], const double UR[3], double nx,
                                             double ny, double g, double F[3]) {
     const double efix = 0.1;
