@@ -128,7 +128,8 @@ struct DevBuf {
 bool all_finite(const double *x, size_t n);
 // Maps the pages of a host array that is about to be written (a fresh array has none: the first
 // write of each page stops in the kernel, on the one thread that writes), on a few host threads for
-// large arrays. Contents are not changed; where the system cannot do it, nothing happens.
+// large arrays; arrays whose pages are there are left alone. Contents are not changed; where the system
+// cannot do it, nothing happens.
 void map_pages(void *p, size_t bytes);
 
 // Captures what `enqueue` queues on `stream` (thread-local capture mode) into an executable

@@ -577,6 +577,27 @@ def test_bounded_grid_barrier_wait_gives_up_and_the_model_stays_usable(monkeypat
     per.close()
 
 
+def test_large_fields_download_whole_into_fresh_used_and_pinned_arrays():
+    """Fields of 32 MB and more (37 MB here): the destination's missing pages are mapped first, whether
+    none, half or all of them are there."""
+    import ctypes as C
+
+    import torch
+    from drifter_b200._abi import check, dptr_array, lib
+    case = configs.c2(nx=48, ny=48, nz=16, order=4, precision="fp64")
+    n3 = case["cfg"].n3
+    assert n3 * 8 > 32 << 20
+    m = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+    m.upload_state(case["q"], case["eta"])
+    half = np.empty(n3)
+    half[: n3 // 2] = 1.0
+    out = [np.empty(n3), half, np.full(n3, np.nan), torch.empty(n3, dtype=torch.float64, pin_memory=True).numpy()]
+    check(lib().drf_dg_download_state(m.handle, dptr_array(out), None, None, None, None, C.byref(C.c_double())))
+    for got, want in zip(out, case["q"]):
+        assert np.array_equal(got, want)
+    m.close()
+
+
 def test_time_copy_leaves_the_state_unchanged():
     case = _tidal_small("mixed", order=4, nx=6, ny=4, nz=4)
     gpu = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
