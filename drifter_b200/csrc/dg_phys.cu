@@ -2511,12 +2511,19 @@ struct drf_dg {
         // has the per-pass kernels' bits with the Lax-Friedrichs flux from N = 2 on (elsewhere the
         // compiler fuses some multiply-add differently, or the flux is hllc_flux_diff).
         if (mixed && G.eos && !(G.flux2d == DRF_FLUX_LF && np >= 3)) return 0;
+        // The launch has a start of its own (it reads its neighbours' state and sets up the traces), which
+        // few subcycles do not pay back: the wide instance takes from three (41 x 41 columns at N = 5: one
+        // 247 us a step in launches per pass and 254 us resident, two 257 and 259 us, four 0.4% slower at
+        // most), the roomy one any number (one within 0.8% or up to 5% faster, two up to 12% faster), but
+        // one at N = 1 (9 x 7 columns: 61.6 and 63.7 us).
+        if (nsub == 1 && np == 2) return 0;
         int form = 0;
         dispatch_np(np, [&](auto npc) {
             constexpr int NP = decltype(npc)::value;
             dispatch_flux(G.flux2d, [&](auto fk) {
                 constexpr int FK = decltype(fk)::value;
-                form = ncol <= resident_columns<NP, FK, false>() ? 1 : (ncol <= resident_columns<NP, FK, true>() ? 2 : 0);
+                form = ncol <= resident_columns<NP, FK, false>() ? 1
+                       : nsub >= 3 && ncol <= resident_columns<NP, FK, true>() ? 2 : 0;
             });
         });
         if (form && !trace.n) {

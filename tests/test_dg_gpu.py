@@ -382,6 +382,24 @@ def test_resident_barotropic_step_equals_per_pass_launches(monkeypatch, order, n
         assert relerr(a[k], b[k]) <= 1e-11, (k, relerr(a[k], b[k]))
 
 
+# where the resident launch gains nothing: one subcycle at N = 1, and fewer than three for a model that
+# fits its wide instance only
+@pytest.mark.parametrize("order,nx,ny,nsub,resident", [(1, 9, 7, 1, False), (1, 9, 7, 2, True), (2, 9, 7, 1, True),
+                                                       (5, 40, 41, 1, False), (5, 40, 41, 2, False),
+                                                       (5, 40, 41, 3, True), (5, 30, 30, 1, True)])
+def test_few_subcycles_take_the_resident_launch_where_it_gains(order, nx, ny, nsub, resident):
+    case = _tidal_small("fp64", order=order, nx=nx, ny=ny, nz=1)
+    dt = case["dt"] * nsub / case["nsub"] * min(1.0, 5.0 / max(nx, ny))
+    m = OceanModel(case["cfg"], case["h"], case["f"], case["taux"], case["tauy"])
+    m.upload_state(case["q"], case["eta"])
+    m.step(dt, nsub, 0)
+    before = launch_count()
+    m.step(dt, nsub, 2)
+    m.sync()
+    assert launch_count() - before == 2 * (7 if resident else 5 + 2 + 2 * nsub)
+    m.close()
+
+
 # the resident launch's roomy instance (9 x 7 columns) and its wide one (counts of 2D nodes between the
 # two instances' room: 57,600 and 102,400 at N = 2, 3; 93,025 at N = 4; 59,040 at N = 5)
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
@@ -417,6 +435,8 @@ def test_one_model_through_all_barotropic_forms(monkeypatch, order, nsub):
         m.upload_state(case["q"], case["eta"])
         models.append(m)
     launches = {None: 7, "1": 6, "0": 5 + 2 + 2 * nsub}
+    if order == 1 and nsub == 1:  # one subcycle at N = 1 keeps a launch per pass
+        launches[None] = launches["0"]
     for k, form in enumerate((None, "1", None, "0", "1", "1", None, None)):
         dt = dt0 * (1.0 - 0.02 * k)
         for m, env in zip(models, (form, "0")):
