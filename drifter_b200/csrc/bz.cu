@@ -1181,7 +1181,9 @@ struct drf_bz {
     int64_t ndof = 0;
     DevBuf<double> dat, Bq, b, bs, x, r, z, p, q, scal, part, mgbuf, coarse;  // b: assembled rhs, bs: rhs of the current solve
     DevBuf<double> diag;  // finest diagonal of Q for the Jacobi steps (formed at first use)
-    DevBuf<int> ctl;
+    // the control words lie behind the scalars, so that one copy reads a residual and them
+    static constexpr int CTL_AT = 16;
+    int *ctl() const { return (int *)(scal.p + CTL_AT); }
     struct Lv {
         DevBuf<double> K, rho, binv, x, b, r;
         ElemOp op;                // K again, by value, for the tile kernel's parameter
@@ -1230,7 +1232,7 @@ struct drf_bz {
     unsigned nparts() const { return 1024; }
     PcgCtl pctl() {
         PcgCtl c;
-        c.sc = scal.p; c.stop = ctl.p; c.iters = ctl.p + 1; c.maxit = ctl.p + 2; c.part = part.p;
+        c.sc = scal.p; c.stop = ctl(); c.iters = ctl() + 1; c.maxit = ctl() + 2; c.part = part.p;
         return c;
     }
 
@@ -1275,7 +1277,7 @@ struct drf_bz {
         PcgCtl c = pctl();
         pcg_head(c);
         int cl[3] = {0, 0, 0};
-        DRF_CUDA(cudaMemcpyAsync(cl, ctl.p, sizeof(cl), cudaMemcpyDeviceToHost, stream));
+        DRF_CUDA(cudaMemcpyAsync(cl, ctl(), sizeof(cl), cudaMemcpyDeviceToHost, stream));
         DRF_CUDA(cudaStreamSynchronize(stream));
         if (cl[0] || cl[1] >= cl[2]) return false;
         mg_apply_reference(r.p, z.p, MG_REF_TOL, MG_REF_MAX_CYCLES, nullptr);
@@ -1557,13 +1559,21 @@ void check_bz(drf_bz *h) { DRF_CHECK(h != nullptr, DRF_E_INVALID, "null smoother
 namespace drf {
 namespace {
 
+// Multigrid iterations to queue without a look: half of those that are left at the rate since the last
+// look (rr0 to rr, squared residuals, in `its` iterations), as the rate grows towards the end
+int unwatched(double rr, double rr0, int its, double target) {
+    if (!(rr < rr0) || !(rr > 0.0)) return 1;
+    const double left = its * std::log(rr / target) / std::log(rr0 / rr);
+    return left > 2.0 ? (int)std::min(0.5 * left, 8.0) : 1;
+}
+
 // PCG on Q x = bs from the x already on the device (bs, x set by the caller); returns the
 // iterations done. Scalars (rr, bb) are left in scal.
 int pcg_run(drf_bz *h, int kind, double tol, int maxit) {
     const int64_t n = h->ndof;
     PcgCtl c = h->pctl();
     const int ctl0[3] = {0, 0, maxit};
-    DRF_CUDA(cudaMemcpyAsync(h->ctl.p, ctl0, sizeof(ctl0), cudaMemcpyHostToDevice, h->stream));
+    DRF_CUDA(cudaMemcpyAsync(h->ctl(), ctl0, sizeof(ctl0), cudaMemcpyHostToDevice, h->stream));
     const double tol2 = tol * tol;
     DRF_CUDA(cudaMemcpyAsync(h->scal.p + S_TOL2, &tol2, 8, cudaMemcpyHostToDevice, h->stream));
     // r = b - Q x ; bb = b.b ; z = M r ; rz = r.z ; p = z
@@ -1594,15 +1604,17 @@ int pcg_run(drf_bz *h, int kind, double tol, int maxit) {
             while (h->pcg_iteration_reference()) {
             }
         int cl[2] = {0, 0};
-        DRF_CUDA(cudaMemcpyAsync(cl, h->ctl.p, sizeof(cl), cudaMemcpyDeviceToHost, h->stream));
+        DRF_CUDA(cudaMemcpyAsync(cl, h->ctl(), sizeof(cl), cudaMemcpyDeviceToHost, h->stream));
         DRF_CUDA(cudaStreamSynchronize(h->stream));
         return cl[1];
     }
     // iterations in graph-captured chunks; converged iterations return early on the device. A
-    // multigrid iteration is worth a look at the stop flag before its V-cycle (0.2 to 1 ms against a
-    // read of about 15 us): the head of the first iteration, then one graph per V-cycle and next head,
-    // so no cycle runs after convergence. In chunks of 8, 6 iterations ran 9 cycles: 64 x 64
-    // elements 2.04 ms a solve against 1.46 ms.
+    // multigrid iteration is worth a look at the stop flag before its V-cycle (0.05 to 1 ms against a
+    // look of 15 to 45 us): the head of the first iteration, then one graph per V-cycle and next head, so
+    // hardly a cycle runs after convergence. In chunks of 8, 6 iterations ran 9 cycles: 64 x 64
+    // elements 2.04 ms a solve against 1.46 ms. A look at every iteration costs more than it saves where
+    // there are many (4 x 4 elements, 14 iterations: 0.89 ms a solve against 0.81 ms in chunks of 8), so
+    // the looks go by the rate (unwatched): 0.78 ms.
     // The learned preconditioner's iterations (0.17 ms at C4, 20 us when they return early) are looked
     // at every 4: C4's 12 iterations 2.07 ms in chunks of 8, 2.02 ms.
     const int chunk = kind == 2 ? 1 : (kind == 3 ? 4 : 8);
@@ -1621,16 +1633,25 @@ int pcg_run(drf_bz *h, int kind, double tol, int maxit) {
             h->graph_chunk = chunk;
         }
         int ctl[2] = {0, 0};
+        double look[drf_bz::CTL_AT + 1 - S_RR];  // the residual to the control words
+        double rr0 = sc[S_RR];
+        int it0 = 0, batch = 1;  // graphs up to the next look
         for (bool head = kind == 2;; head = false) {
-            if (head) {
-                h->pcg_head(c);
-            } else {
-                DRF_CUDA(cudaGraphLaunch(h->graph, h->stream));
-                launch_counter().fetch_add(h->graph_kernels);
-            }
-            DRF_CUDA(cudaMemcpyAsync(ctl, h->ctl.p, sizeof(ctl), cudaMemcpyDeviceToHost, h->stream));
+            if (head) h->pcg_head(c);
+            else
+                for (int k = 0; k < batch; ++k) {
+                    DRF_CUDA(cudaGraphLaunch(h->graph, h->stream));
+                    launch_counter().fetch_add(h->graph_kernels);
+                }
+            DRF_CUDA(cudaMemcpyAsync(look, h->scal.p + S_RR, sizeof(look), cudaMemcpyDeviceToHost, h->stream));
             DRF_CUDA(cudaStreamSynchronize(h->stream));
+            std::memcpy(ctl, look + drf_bz::CTL_AT - S_RR, sizeof(ctl));
             if (ctl[0] || ctl[1] >= maxit) break;
+            if (kind == 2) {
+                batch = std::min(unwatched(look[0], rr0, ctl[1] - it0, tol2 * sc[S_BB]), maxit - ctl[1]);
+                rr0 = look[0];
+                it0 = ctl[1];
+            }
         }
         it = ctl[1];
     }
@@ -1891,10 +1912,9 @@ int drf_bz_create(const drf_bz_grid_desc *g, const double *dgauss, drf_bz **out)
         DRF_CUDA(cudaMemcpy(h->dat.p, dgauss, nd * 8, cudaMemcpyHostToDevice));
         up(h->Bq, h->H.Bq);
         for (auto *v : {&h->b, &h->bs, &h->x, &h->r, &h->z, &h->p, &h->q}) v->alloc(h->ndof);
-        h->scal.alloc(S_NSLOT);
+        h->scal.alloc(drf_bz::CTL_AT + 2);
         // per-block partials: the fused apply-dot writes one value per apply block
         h->part.alloc(std::max<size_t>(4096, (size_t)nblk(h->ndof) + 16));
-        h->ctl.alloc(3);
         h->form_diag();
         bz_rhs_kernel<<<nblk(h->ndof), BS, 0, h->stream>>>(F.n, F.nd, h->dat.p, h->Bq.p, g->lambda, h->b.p);
         DRF_LAUNCHED();

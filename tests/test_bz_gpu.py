@@ -67,6 +67,28 @@ def test_vcycle_color_steps_at_tile_edges(n, coarsest, pre, post):
     assert relres < 1e-6 and k < 100
 
 
+@pytest.mark.parametrize("n,lam", [(4, 1e-2), (16, 1.0), (16, 1e-2)])
+def test_multigrid_iterations_queued_between_looks_stop_where_they_should(n, lam):
+    """Iterations queued without a look at the stop flag end at the iteration limit and at convergence
+    (5 to some 30 iterations here): counts as asked for, residuals that belong to them, and the
+    limit at the full count leaves the very solution of a solve without one."""
+    g, _ = pair(n, lam=lam)
+    g.mg_setup(2)
+    x, info = g.solve("mg", tol=1e-10, maxit=1000)
+    assert 4 <= info["iters"] < 60
+    b = g.rhs()
+    last = 1.0
+    for k in range(1, info["iters"] + 1):
+        xk, ik = g.solve("mg", tol=1e-10, maxit=k)
+        assert ik["iters"] == k
+        true = np.linalg.norm(b - g.apply_Q(xk)) / np.linalg.norm(b)
+        assert abs(ik["relres"] - true) <= 0.1 * true + 1e-9  # the recurrence against the true residual
+        last = ik["relres"]
+    assert last == info["relres"] and np.array_equal(xk, x)
+    x0, i0 = g.solve("mg", tol=1e-300, maxit=info["iters"] + 3)
+    assert i0["iters"] == info["iters"] + 3 and i0["relres"] <= 1e-9
+
+
 @pytest.mark.parametrize("before", [None, 4])
 def test_multigrid_setup_that_finds_no_memory_leaves_the_operator(before):
     """drf_mg_setup on a full device returns DRF_E_NOMEM; the smoother, with no hierarchy or one of
