@@ -1803,7 +1803,7 @@ __global__ void BARO_BOUNDS baro_subcycles_kernel(const __grid_constant__ BaroAr
 // resident) and every poll is bounded.
 //
 // Bound by latency: an exchange and the dependent chain of a face flux (a reciprocal, a square
-// root) per pass, 1.5 us at C1 (256 columns, N = 3) against 3.3 us for a launch per pass.
+// root) per pass, 1.5 us at C1 (256 columns, N = 3) against 2.8 us for a launch per pass.
 struct ResidentArgs {
     double dt, dtb;
     int nsub, ncol;
@@ -2499,8 +2499,8 @@ struct drf_dg {
 
     // Whether the barotropic step takes the resident form (0 no, 1 roomy, 2 wide): where the
     // model fits it, as one launch then replaces 2 nsub + 1 and a pass costs one exchange of
-    // traces instead of a launch (per step, both measured: C1 198 -> 126 us, 23 x 17 columns at
-    // N = 2 with HLLC 280 -> 184 us, 64 x 64 at N = 4 1221 -> 1139 us). Launch forms fixed by
+    // traces instead of a launch (per step, both measured, the launches overlapped: C1 178 -> 124 us,
+    // 23 x 17 columns at N = 2 with HLLC 261 -> 183 us, 64 x 64 x 16 at N = 4 1189 -> 1140 us). Forms fixed by
     // DRIFTER_B200_TUNE=0 or DRIFTER_B200_BARO_PERSISTENT stay as they are.
     int resident_form(int nsub) {
         const char *tu = std::getenv("DRIFTER_B200_TUNE"), *pe = std::getenv("DRIFTER_B200_BARO_PERSISTENT");
@@ -2810,7 +2810,9 @@ void drf_dg::setup(const drf_mesh_desc *mesh, const drf_dg_params *params, const
 // Autotuner of the barotropic tile (water columns per CTA of the subcycle kernels): times the
 // predictor kernel, which writes only scratch arrays, at every candidate tile on the model's
 // stream (two warm-up launches, then ten between CUDA events) and keeps the fastest. Choices
-// are cached per (device, order, flux, number of columns) for the life of the process.
+// are cached per (device, order, flux, number of columns) for the life of the process. The launches
+// timed follow one another; in the step they overlap, which the candidates share. A model in the
+// resident form uses the tile for its forcing pass only.
 // DRIFTER_B200_TUNE=0 in the environment keeps the default tile.
 void drf_dg::tune_baro() {
     if (baro_cpb) return;

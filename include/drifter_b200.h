@@ -187,10 +187,12 @@ int drf_dg_set_forcing(drf_dg *m, const double *taux, const double *tauy);
 /* Copies the 2D surface elevation to the host (synchronous). */
 int drf_dg_download_surface(drf_dg *m, double *eta);
 
-/* Autotuned launch shape: the barotropic subcycle kernels' tile (water columns per CTA) chosen
- * by timing the candidates 2, 4, 8, 16 on this model (done at the first step, or here), and
- * the candidates' times in ms (baro_ms4 may be NULL). No counterpart in the reference, which
- * has no kernels; DRIFTER_B200_TUNE=0 keeps the default tile of 8. */
+/* Autotuned launch shape: the tile (water columns per CTA) of the barotropic launches per pass,
+ * chosen by timing the predictor kernel at the candidates 2, 4, 8, 16 on this model, launch after
+ * launch (done at the first step, or here), and the candidates' times in ms (baro_ms4 may be NULL).
+ * A model whose subcycles run in one resident launch uses it for its forcing pass only. No
+ * counterpart in the reference, which has no kernels; DRIFTER_B200_TUNE=0 keeps the default tile of
+ * 8 and a launch per pass. */
 int drf_dg_tuning(drf_dg *m, int *baro_cols_per_cta, double *baro_ms4);
 /* Autotuned stage launch: how far ahead (in half waves of resident CTAs, 0..2, and in columns)
  * each stage CTA prefetches a later column into L2, chosen by timing the three on this model (at
